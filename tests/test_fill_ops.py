@@ -172,6 +172,34 @@ def test_aa_fill_matches_aa_fill_cpu(backend, oracle, fill_cases, rule):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("w,h,n", [(1, 1, 3), (3, 5, 9), (63, 4, 40), (1023, 3, 60), (1024, 5, 60), (1025, 4, 200),
+                                   (2051, 3, 400), (130, 5, 1100), (1100, 2, 1400)])
+def test_aa_fill_chunk_edges(backend, oracle, w, h, n):
+    """Widths around the 1,024-column chunk, rows around the band of 4, lines of more crossings than a list keeps
+    (column buckets) and more segments than a band keeps; crossings at pixel samples, off the window and at infinity."""
+    rng = np.random.default_rng(w * 7 + n)
+    segs = np.stack([rng.uniform(-0.2, 1.2, n) * w, rng.uniform(-1, h + 1, n), rng.uniform(-0.2, 1.2, n) * w,
+                     rng.uniform(-1, h + 1, n)], 1).astype(np.float32)
+    k = n // 3
+    segs[:k] = np.floor(segs[:k] * 2) / 2  # corners on samples' grid
+    segs[0] = (np.inf, 0, np.inf, h)
+    segs[1] = (-np.inf, h, -np.inf, 0)
+    segs[2] = (np.nan, 0, 1, h)
+    for rule in (0, 1):
+        exp = oracle.aa_fill_cpu(segs, 0.0, 0.0, w, h, eo=bool(rule))
+        sb, cb = _dev(backend, segs), backend.alloc_device(w * h + 1)
+        try:
+            backend.upload_async(cb, np.full(w * h + 1, 77, np.uint8))
+            _run(backend, lambda: backend.record_aa_fill(sb, n, cb, w, h, rule))
+            got = np.empty(w * h + 1, np.uint8)
+            backend.wait_download(backend.download_async(cb, got))
+            assert np.array_equal(got[:-1], exp.ravel()) and got[-1] == 77
+        finally:
+            backend.free_device(sb)
+            backend.free_device(cb)
+
+
+@pytest.mark.gpu
 def test_aa_fill_without_segments_is_zero(backend):
     cb = backend.alloc_device(40 * 30)
     sb = backend.alloc_device(16)
