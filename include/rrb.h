@@ -448,7 +448,9 @@ int rrb_get_tuning(rrb_ctx* ctx, rrb_tuning* t);
 /* Counters of the last recorded batch (filled after the page fence). */
 typedef struct {
     uint64_t paths, pieces, segments;       /* input paths, walk pieces, flattened segments */
-    uint64_t aa_rows, spans, row_overflows; /* AA rows built, spans emitted, rows on the slow path */
+    uint64_t aa_rows, spans, row_overflows; /* AA rows of the paths, spans emitted, rows on the slow path (rows
+                                               that later full-tile layers hide everywhere are not built and are
+                                               in neither of the last two, nor in nonterminating_rows) */
     uint64_t tiles, tile_pairs;             /* tiles with work, (tile, path) pairs */
     uint64_t nonterminating_rows;           /* rows whose winding never returns to 0 */
     uint64_t kernel_launches;               /* kernels launched by the last record call */

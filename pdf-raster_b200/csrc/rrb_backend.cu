@@ -71,7 +71,8 @@ struct rrb_ctx {
     // Batch scratch.
     Scratch s_pts, s_flags, s_off, s_rule, s_gray, s_alpha, s_page, s_geom, s_pw, s_ph, s_mtx;
     Scratch s_pieces, s_clip, s_edge_off, s_edges, s_info, s_rows, s_chunks, s_super_cnt, s_super_list;
-    Scratch s_super_start;  // per supertile: one past its last opaque full layer
+    Scratch s_tile_start;   // per tile: the list position where its compositing starts
+    Scratch s_chunk_live;   // per row chunk: some tile reads it
     Scratch s_big;          // piece slots of curves flattened by a warp each
     Scratch s_lanes;        // per big curve: each lane's segment count (u8 x 32), from the count pass
     Scratch s_row_idx, s_spans, s_ovf, s_scratch, s_ctr, s_block, s_stats, s_groups, s_slots, s_path_pieces, s_ovf2;
@@ -252,11 +253,11 @@ int launch_composite(rrb_ctx* c, int tw, int th, int grid, const PathInfo* info,
                      uint32_t n_pages, uint32_t n_tiles, const uint32_t* super_off, const uint32_t* super_list,
                      const uint32_t* row_off, const uint2* row_idx, const uint32_t* spans, const int4* runs,
                      uint8_t* arena, int rowmap, BatchCounters* ctr, const uint32_t* path_rgb,
-                     bool rectilinear, const uint32_t* super_start) {
+                     bool rectilinear, const uint32_t* tile_start) {
 #define RRB_COMP(TW, TH, RGB, FEW)                                                                           \
     k_composite<TW, TH, RGB, FEW><<<grid, comp_threads(TW, TH), 0, c->stream>>>(                              \
         info, geom, n_pages, n_tiles, SUPER, SUPER, super_off, super_list, row_off, row_idx, spans, runs, arena, \
-        rowmap, ctr, path_rgb, super_start)
+        rowmap, ctr, path_rgb, tile_start)
 #define RRB_COMP_SHAPE(RGB, FEW)                                  \
     do {                                                          \
         if (tw == 64 && th == 16) RRB_COMP(64, 16, RGB, FEW);     \
@@ -727,7 +728,7 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
     stage(c, 6);
     k_super_bin<false><<<grid_for(c, supers * 32, 256), 256, 0, c->stream>>>(
         as<PathInfo>(c->s_info), as<PageGeom>(B->geom), n_pages, NSUP, SUPER, SUPER, as<uint32_t>(c->s_super_cnt),
-        nullptr, nullptr, nullptr);
+        nullptr, nullptr);
     c->launches += 1;
     stage_end(c, 6);
     RRB_CUDA(c, cudaGetLastError());
@@ -786,22 +787,35 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
     if ((rc = ensure(c, c->s_ovf, std::max<uint64_t>(1, n_groups) * sizeof(uint2)))) return rc;
     if ((rc = ensure(c, c->s_super_list, std::max<uint64_t>(1, n_pairs) * sizeof(uint32_t)))) return rc;
     if ((rc = ensure(c, c->s_runs, std::max<uint64_t>(1, n_runs) * sizeof(int4)))) return rc;
-    const PageGeom& last_page = B->geom_h[n_pages - 1];
-    const uint64_t n_super_tiles =
-        last_page.super_base + static_cast<uint64_t>(last_page.nsx) * ((last_page.h + SUPER - 1) / SUPER);
-    if ((rc = ensure(c, c->s_super_start, n_super_tiles * sizeof(uint32_t)))) return rc;
-    RRB_CUDA(c, cudaMemsetAsync(c->s_super_start.p, 0, n_super_tiles * sizeof(uint32_t), c->stream));
+    if ((rc = ensure(c, c->s_tile_start, tiles * sizeof(uint32_t)))) return rc;
+    if ((rc = ensure(c, c->s_chunk_live, std::max<uint64_t>(1, n_chunks)))) return rc;
+    RRB_CUDA(c, cudaMemsetAsync(c->s_chunk_live.p, 0, std::max<uint64_t>(1, n_chunks), c->stream));
     stage(c, 8);
     k_super_bin<true><<<grid_for(c, supers * 32, 256), 256, 0, c->stream>>>(
         as<PathInfo>(c->s_info), as<PageGeom>(B->geom), n_pages, NSUP, SUPER, SUPER, nullptr,
-        as<uint32_t>(c->s_super_cnt), as<uint32_t>(c->s_super_list), as<uint32_t>(c->s_super_start));
+        as<uint32_t>(c->s_super_cnt), as<uint32_t>(c->s_super_list));
+    c->launches += 1;
+    if (n_runs) {  // before k_tile_start, which reads the solid boxes
+        k_recti<true><<<grid_for(c, n_paths, 128, 16), 128, 0, c->stream>>>(
+            as<PathInfo>(c->s_info), NP, as<Edge>(c->s_edges), as<uint32_t>(B->pw), rowmap, nullptr,
+            as<uint32_t>(c->s_run_off), as<int4>(c->s_runs), as<uint32_t>(c->s_spans), static_cast<uint32_t>(cell_cap),
+            as<BatchCounters>(c->s_ctr), pclip);
+        c->launches += 1;
+    }
+    k_tile_start<<<grid_for(c, tiles * 32, START_WARPS * 32), START_WARPS * 32, 0, c->stream>>>(
+        as<PathInfo>(c->s_info), as<PageGeom>(B->geom), n_pages, static_cast<uint32_t>(tiles), static_cast<int>(tw),
+        static_cast<int>(th), SUPER, SUPER, as<uint32_t>(c->s_super_cnt), as<uint32_t>(c->s_super_list), rowmap,
+        B->bpp == 3, as<uint32_t>(c->s_chunks), as<uint32_t>(c->s_tile_start), as<uint8_t>(c->s_chunk_live),
+        as<BatchCounters>(c->s_ctr));
     c->launches += 1;
     stage_end(c, 8);
+    RRB_CUDA(c, cudaGetLastError());
     stage(c, 9);
     if (n_chunks) {
-        if ((rc = ensure(c, c->s_chunk_path, n_chunks * sizeof(uint32_t)))) return rc;
-        k_chunk_paths<<<grid_for(c, n_paths * 32, 256), 256, 0, c->stream>>>(as<uint32_t>(c->s_chunks), NP,
-                                                                            as<uint32_t>(c->s_chunk_path));
+        if ((rc = ensure(c, c->s_chunk_path, n_chunks * sizeof(uint2)))) return rc;
+        k_chunk_paths<<<grid_for(c, n_paths * 32, 256), 256, 0, c->stream>>>(
+            as<uint32_t>(c->s_chunks), NP, as<uint8_t>(c->s_chunk_live), as<uint2>(c->s_chunk_path),
+            as<BatchCounters>(c->s_ctr));
         c->launches += 1;
         // Shapes of the row stage: 12 list entries per AA row with 8 warps per
         // block (the default), 16 entries with 4 warps (fewer rows go to
@@ -812,9 +826,9 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
                                              static_cast<int>(smem)));
             kernel<<<grid_for(c, n_chunks * 32, warps * 32, 16), warps * 32, smem, c->stream>>>(
                 as<PathInfo>(c->s_info), as<uint32_t>(c->s_chunks), as<uint32_t>(c->s_rows), as<Edge>(c->s_edges),
-                gmin, gmax, as<uint32_t>(B->pw), NP, as<uint2>(c->s_row_idx), as<uint32_t>(c->s_spans),
+                gmin, gmax, as<uint32_t>(B->pw), as<uint2>(c->s_row_idx), as<uint32_t>(c->s_spans),
                 static_cast<uint32_t>(cell_cap), as<uint2>(c->s_ovf), static_cast<uint32_t>(std::max<uint64_t>(1, n_groups)),
-                as<BatchCounters>(c->s_ctr), as<uint32_t>(c->s_chunk_path), pclip);
+                as<BatchCounters>(c->s_ctr), as<uint2>(c->s_chunk_path), pclip);
             return RRB_OK;
         };
         switch (B->row_shape) {
@@ -825,13 +839,6 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
             default: rc = rows(k_rows<KCAP, ROWS_WARPS>, ROWS_WARPS, rows_smem_bytes<KCAP, ROWS_WARPS>());
         }
         if (rc) return rc;
-        c->launches += 1;
-    }
-    if (n_runs) {
-        k_recti<true><<<grid_for(c, n_paths, 128, 16), 128, 0, c->stream>>>(
-            as<PathInfo>(c->s_info), NP, as<Edge>(c->s_edges), as<uint32_t>(B->pw), rowmap, nullptr,
-            as<uint32_t>(c->s_run_off), as<int4>(c->s_runs), as<uint32_t>(c->s_spans), static_cast<uint32_t>(cell_cap),
-            as<BatchCounters>(c->s_ctr), pclip);
         c->launches += 1;
     }
     if (B->has_hairline && hl_rows) {
@@ -930,7 +937,7 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
                                as<uint32_t>(c->s_super_cnt), as<uint32_t>(c->s_super_list), as<uint32_t>(c->s_rows),
                                as<uint2>(c->s_row_idx), as<uint32_t>(c->s_spans), as<int4>(c->s_runs), arena,
                                rowmap, as<BatchCounters>(c->s_ctr), B->bpp == 3 ? as<uint32_t>(B->rgb) : nullptr,
-                               n_runs > 0, as<uint32_t>(c->s_super_start))))
+                               n_runs > 0, as<uint32_t>(c->s_tile_start))))
         return rc;
     stage_end(c, 11);
     c->stats.paths = n_paths;
@@ -1018,7 +1025,7 @@ void set_binning(std::vector<PageGeom>& geom, uint64_t& supers_out) {
 void release_scratch(rrb_ctx* c) {
     cudaStreamSynchronize(c->stream);
     Scratch* all[] = {&c->s_pieces, &c->s_clip, &c->s_edge_off, &c->s_edges, &c->s_info, &c->s_rows, &c->s_chunks,
-                      &c->s_super_cnt, &c->s_super_list, &c->s_super_start, &c->s_big, &c->s_lanes, &c->s_row_idx, &c->s_spans, &c->s_ovf, &c->s_scratch,
+                      &c->s_super_cnt, &c->s_super_list, &c->s_tile_start, &c->s_chunk_live, &c->s_big, &c->s_lanes, &c->s_row_idx, &c->s_spans, &c->s_ovf, &c->s_scratch,
                       &c->s_groups, &c->s_slots, &c->s_path_pieces, &c->s_ovf2, &c->s_run_off, &c->s_runs,
                       &c->s_chunk_path, &c->s_clip_lo, &c->s_hl_clip};
     for (Scratch* x : all) {
@@ -1701,7 +1708,7 @@ int rrb_destroy(rrb_ctx* c) {
     cudaStreamSynchronize(c->stream);
     Scratch* all[] = {&c->s_pts, &c->s_flags, &c->s_off, &c->s_rule, &c->s_gray, &c->s_alpha, &c->s_page,
                       &c->s_geom, &c->s_pw, &c->s_ph, &c->s_mtx, &c->s_pieces, &c->s_clip, &c->s_edge_off,
-                      &c->s_edges, &c->s_info, &c->s_rows, &c->s_chunks, &c->s_super_cnt, &c->s_super_list, &c->s_super_start, &c->s_big, &c->s_lanes,
+                      &c->s_edges, &c->s_info, &c->s_rows, &c->s_chunks, &c->s_super_cnt, &c->s_super_list, &c->s_tile_start, &c->s_chunk_live, &c->s_big, &c->s_lanes,
                       &c->s_row_idx, &c->s_spans, &c->s_ovf, &c->s_scratch, &c->s_ctr, &c->s_block, &c->s_stats,
                       &c->s_groups, &c->s_slots, &c->s_path_pieces, &c->s_ovf2, &c->s_run_off, &c->s_runs,
                       &c->s_chunk_path, &c->s_clip_lo};
