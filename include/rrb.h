@@ -215,10 +215,11 @@ typedef struct {
  * operation in IEEE f32 as written. A tile whose record range runs past the
  * records buffer is filled as empty. */
 int rrb_record_tile_fill(rrb_ctx* ctx, const rrb_tile_fill_params* p);
-/* tile_fill from segments: the tile records are built on the device
- * (build_tile_records, crates/gpu/src/fill.rs:82-264, with a stable key
- * sort) and kept in the context's scratch. Synchronises once, to size the
- * records; *n_records (optional) receives their count. */
+/* tile_fill from segments: the tile records are those of build_tile_records
+ * (crates/gpu/src/fill.rs:82-264, with a stable key sort), formed on the
+ * device. *n_records (optional) receives their count: the call then waits on
+ * the stream once (more than 32,768 segments: once in any case, to size the
+ * records, which are kept in the context's scratch). */
 int rrb_record_tile_fill_segs(rrb_ctx* ctx, const rrb_aa_fill_params* p, uint64_t* n_records);
 
 /* GpuBackend::record_scan (crates/gpu/src/backend/mod.rs:340-353; ScanParams

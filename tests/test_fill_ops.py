@@ -255,6 +255,35 @@ def test_tile_fill_from_segments_matches_oracle(backend, oracle, fill_cases, rul
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("w,h,n", [(1, 1, 2), (16, 16, 1023), (17, 15, 1024), (256, 33, 1025), (257, 16, 2500),
+                                   (500, 20, 5000), (100, 70, 32768), (100, 70, 32769)])
+def test_tile_fill_segs_scan_edges(backend, oracle, w, h, n):
+    """Both routes of tile_fill from segments: the ordered scan up to 32,768 segments (chunks of 1,024, lists that fill
+    up in one tile row, groups of 16 tiles) and the sorted records beyond; sums of many records per pixel in order."""
+    rng = np.random.default_rng(w + n)
+    segs = np.stack([rng.uniform(-0.2, 1.2, n) * w, rng.uniform(-2, h + 2, n), rng.uniform(-0.2, 1.2, n) * w,
+                     rng.uniform(-2, h + 2, n)], 1).astype(np.float32)
+    segs[: n // 4, 2:] = segs[: n // 4, :2] + rng.normal(0, 1.5, (n // 4, 2))
+    segs[n // 4: n // 2] = np.round(segs[n // 4: n // 2])  # corners on pixel and tile edges
+    segs[0], segs[1] = (np.nan, 0, 1, h), (0, np.inf, 1, 2)
+    recs, starts, counts, gw = oracle.build_tile_records(segs, 0.0, 0.0, w, h)
+    for rule in (0, 1):
+        exp = oracle.tile_fill(recs, starts, counts, gw, w, h, eo=bool(rule))
+        sb, cb = _dev(backend, segs), backend.alloc_device(w * h + 1)
+        try:
+            backend.upload_async(cb, np.full(w * h + 1, 77, np.uint8))
+            out = {}
+            _run(backend, lambda: out.setdefault("n", backend.record_tile_fill_segs(sb, n, cb, w, h, rule)))
+            assert out["n"] == len(recs)
+            got = np.empty(w * h + 1, np.uint8)
+            backend.wait_download(backend.download_async(cb, got))
+            assert np.array_equal(got[:-1], exp.ravel()) and got[-1] == 77
+        finally:
+            backend.free_device(sb)
+            backend.free_device(cb)
+
+
+@pytest.mark.gpu
 def test_tile_fill_range_past_the_records_is_an_empty_tile(backend, oracle):
     segs = np.asarray(rect(2, 2, 30, 30), np.float32).reshape(-1, 4)
     recs, starts, counts, gw = oracle.build_tile_records(segs, 0.0, 0.0, 32, 32)
