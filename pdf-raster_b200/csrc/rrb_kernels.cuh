@@ -1250,6 +1250,24 @@ __device__ __forceinline__ int gather_row(const PathInfo& P, int32_t lo, int32_t
     return n;
 }
 
+// The winding walk of a lane's sorted list; its union of spans replaces it in place.
+template <int LS>
+__device__ __forceinline__ int walk_list(int n, int32_t mask, int32_t aa_width, int32_t lo, int32_t hi, int32_t* x0s,
+                                         int32_t* x1s, int32_t* cns, int lane, uint32_t& nonterm) {
+    return walk_row(
+        n, mask, aa_width, lo, hi,
+        [&](int i, int32_t& x0, int32_t& x1, int32_t& cc) {
+            x0 = x0s[i * LS + lane];
+            x1 = x1s[i * LS + lane];
+            cc = cns[i * LS + lane];
+        },
+        [&](int k, int32_t s0, int32_t e0) {
+            x0s[k * LS + lane] = s0;
+            x1s[k * LS + lane] = e0;
+        },
+        nonterm);
+}
+
 // sort_unstable_by_key(x0) on a lane's list (stable insertion sort, as Rust
 // std sorts slices of up to 20 elements) followed by the render_aa_line
 // winding walk; the row's union of spans replaces the list in place.
@@ -1270,18 +1288,7 @@ __device__ __forceinline__ int sort_and_walk(int n, int32_t mask, int32_t aa_wid
         x1s[b * LS + lane] = t1;
         cns[b * LS + lane] = tc;
     }
-    return walk_row(
-        n, mask, aa_width, lo, hi,
-        [&](int i, int32_t& x0, int32_t& x1, int32_t& cc) {
-            x0 = x0s[i * LS + lane];
-            x1 = x1s[i * LS + lane];
-            cc = cns[i * LS + lane];
-        },
-        [&](int k, int32_t s0, int32_t e0) {
-            x0s[k * LS + lane] = s0;
-            x1s[k * LS + lane] = e0;
-        },
-        nonterm);
+    return walk_list<LS>(n, mask, aa_width, lo, hi, x0s, x1s, cns, lane, nonterm);
 }
 
 // The row chunks to build, (chunk, its path): all of them in order, or, when
@@ -1700,9 +1707,50 @@ __global__ void k_recti(PathInfo* __restrict__ info, uint32_t n_paths, const Edg
 
 // Pixel rows whose sub-row lists overflowed KCAP: one warp per pixel row
 // (lanes 0-3 = its AA rows) with MID_K entries per row in shared memory.
-// Rows longer than that go to k_groups_slow through ovf2.
+// Rows longer than that go to k_groups_slow through ovf2. The four lists are
+// sorted by the whole warp, each entry counting those before it: an insertion
+// sort by the row's own lane takes n^2 / 4 steps of shared-memory latency (a
+// row of 128 entries: 125 us), this n / 32 x n of one instruction each.
 constexpr int MID_K = 128;
 constexpr int MID_WARPS = 4;
+
+// Stable sort by x0 of the first n <= MID_K entries of column q of lists with
+// LS columns, by a warp.
+template <int LS>
+__device__ __forceinline__ void warp_rank_sort(int n, int q, int32_t* x0s, int32_t* x1s, int32_t* cns, int lane) {
+    constexpr int PER = MID_K / 32;
+    int32_t x0[PER], x1[PER], cc[PER];
+    int rank[PER];
+    bool unsorted = false;
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+        const int i = lane + 32 * u;
+        rank[u] = 0;
+        if (i < n) {
+            x0[u] = x0s[i * LS + q];
+            x1[u] = x1s[i * LS + q];
+            cc[u] = cns[i * LS + q];
+            unsorted |= i > 0 && x0s[(i - 1) * LS + q] > x0[u];
+        }
+    }
+    if (!__any_sync(0xffffffffu, unsorted)) return;
+    for (int j = 0; j < n; ++j) {
+        const int32_t xj = x0s[j * LS + q];
+#pragma unroll
+        for (int u = 0; u < PER; ++u)
+            if (32 * u < n) rank[u] += (xj < x0[u] || (xj == x0[u] && j < lane + 32 * u)) ? 1 : 0;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+        if (lane + 32 * u < n) {
+            x0s[rank[u] * LS + q] = x0[u];
+            x1s[rank[u] * LS + q] = x1[u];
+            cns[rank[u] * LS + q] = cc[u];
+        }
+    }
+    __syncwarp();
+}
 
 __global__ void __launch_bounds__(MID_WARPS * 32) k_groups_mid(
     const PathInfo* __restrict__ info, const uint32_t* __restrict__ group_off, const Edge* __restrict__ edges,
@@ -1731,8 +1779,13 @@ __global__ void __launch_bounds__(MID_WARPS * 32) k_groups_mid(
         const bool overflow = valid && n > MID_K;
         int ns = 0;
         const int2 cx = path_clip ? make_int2(path_clip[p].x, path_clip[p].y) : make_int2(0, aa_width);
+        __syncwarp();
+        for (int q = 0; q < 4; ++q) {
+            const int nq = __shfl_sync(0xffffffffu, (valid && !overflow) ? n : 0, q);
+            if (nq > 1) warp_rank_sort<4>(nq, q, sx0[w], sx1[w], scn[w], lane);
+        }
         if (valid && !overflow)
-            ns = sort_and_walk<4>(n, mask, aa_width, cx.x, cx.y, sx0[w], sx1[w], scn[w], lane, nonterm);
+            ns = walk_list<4>(n, mask, aa_width, cx.x, cx.y, sx0[w], sx1[w], scn[w], lane, nonterm);
         if (lane < 4) sns[w][lane] = (valid && !overflow) ? ns : 0;
         const bool any_ovf = __any_sync(0xffffffffu, overflow);
         __syncwarp();
@@ -1770,6 +1823,53 @@ __global__ void __launch_bounds__(MID_WARPS * 32) k_groups_mid(
 // path's edge count.
 constexpr int SLOW_WARPS = 4;  // warps per block of k_groups_slow
 
+// Stable sort by x0 of n entries (a row of more than 20 entries: see the tie
+// note in the oracle) by a warp, through the temporary T: blocks of 32 by rank
+// in registers, then merges in which each entry finds its place by a binary
+// search of the other run (runs on the left come first among equals). Skipped
+// when the entries already come in order.
+__device__ __forceinline__ void warp_merge_sort(int3* L, int3* T, int n, uint32_t lane) {
+    bool unsorted = false;
+    for (int i = 1 + static_cast<int>(lane); i < n; i += 32) unsorted |= L[i - 1].x > L[i].x;
+    if (!__any_sync(0xffffffffu, unsorted)) return;
+    for (int b = 0; b < n; b += 32) {
+        const int i = b + static_cast<int>(lane);
+        const int3 e = i < n ? L[i] : make_int3(INT32_MAX, 0, 0);
+        int rank = 0;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            const int32_t xj = __shfl_sync(0xffffffffu, e.x, j);
+            rank += (xj < e.x || (xj == e.x && j < static_cast<int>(lane))) ? 1 : 0;  // lanes past n stay last
+        }
+        if (i < n) T[b + rank] = e;
+    }
+    __syncwarp();
+    int3 *A = T, *B = L;
+    for (int w = 32; w < n; w *= 2) {
+        for (int i = lane; i < n; i += 32) {
+            const int lo = i / (2 * w) * (2 * w), mid = min(lo + w, n), hi = min(lo + 2 * w, n);
+            const int3 e = A[i];
+            const bool left = i < mid;
+            int a = left ? mid : lo, z = left ? hi : mid;  // the other run
+            const int from = a;
+            while (a < z) {
+                const int m = (a + z) >> 1;
+                const int32_t x = A[m].x;
+                if (left ? x < e.x : x <= e.x) a = m + 1;
+                else z = m;
+            }
+            B[lo + (i - (left ? lo : mid)) + (a - from)] = e;
+        }
+        __syncwarp();
+        int3* t = A;
+        A = B;
+        B = t;
+    }
+    if (A != L)
+        for (int i = lane; i < n; i += 32) L[i] = A[i];
+    __syncwarp();
+}
+
 __global__ void k_groups_slow(const PathInfo* __restrict__ info, const uint32_t* __restrict__ group_off,
                               const Edge* __restrict__ edges, const int32_t* __restrict__ gmin,
                               const int32_t* __restrict__ gmax, const uint32_t* __restrict__ page_w,
@@ -1780,8 +1880,8 @@ __global__ void k_groups_slow(const PathInfo* __restrict__ info, const uint32_t*
     // at a time (aligned groups whose row bounds miss the row are skipped) and
     // stages each lane's entries for the four AA sub-rows in shared memory;
     // lanes 0-3 then fold them, in edge order, into their sub-row's list
-    // (merging into the list's last entry as fill_intersections does). Lane 0
-    // sorts, walks and writes the cells.
+    // (merging into the list's last entry as fill_intersections does). The
+    // warp sorts the lists, lanes 0-3 walk them, lane 0 writes the cells.
     __shared__ int3 stage[SLOW_WARPS][4][32];
     const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const uint32_t n_ovf = min(ctr->ovf2_count, ovf_cap);
@@ -1856,52 +1956,33 @@ __global__ void k_groups_slow(const PathInfo* __restrict__ info, const uint32_t*
           }
         }
         if (lane < 4 && has_last) Ls[n_s++] = last;
+        __syncwarp();
+        for (int sub = 0; sub < 4; ++sub)
+            warp_merge_sort(scratch + sb + static_cast<uint32_t>(sub) * ne, scratch + sb + 4u * ne,
+                            __shfl_sync(0xffffffffu, n_s, sub), lane);
+        // Each lane of the first four walks its sub-row's sorted list.
+        if (lane < 4) {
+            const int32_t r = 4 * g + static_cast<int32_t>(lane);
+            n_s = r < P.y0 || r > P.y1 ? 0
+                                       : walk_row(
+                                             n_s, mask, aa_width, cx.x, cx.y,
+                                             [&](int i, int32_t& x0, int32_t& x1, int32_t& cc) {
+                                                 const int3 v = Ls[i];
+                                                 x0 = v.x;
+                                                 x1 = v.y;
+                                                 cc = v.z;
+                                             },
+                                             [&](int q, int32_t s0, int32_t e0) {
+                                                 Ls[q].x = s0;
+                                                 Ls[q].y = e0;
+                                             },
+                                             nonterm);
+        }
         int n4[4];
 #pragma unroll
         for (int sub = 0; sub < 4; ++sub) n4[sub] = __shfl_sync(0xffffffffu, n_s, sub);
         __syncwarp();
         if (lane != 0) continue;
-        for (int sub = 0; sub < 4; ++sub) {
-            const int32_t r = 4 * g + sub;
-            if (r < P.y0 || r > P.y1) continue;
-            int3* L = scratch + sb + static_cast<uint32_t>(sub) * ne;
-            int n = n4[sub];
-            // Stable sort by x0 (a row of more than 20 entries: see the tie
-            // note in the oracle): bottom-up merge sort through the temporary
-            // list, skipped when the entries already come in order.
-            bool sorted = true;
-            for (int a = 1; a < n && sorted; ++a) sorted = L[a - 1].x <= L[a].x;
-            if (!sorted) {
-                int3* A = L;
-                int3* T = scratch + sb + 4u * ne;
-                for (int w = 1; w < n; w *= 2) {
-                    for (int lo = 0; lo < n; lo += 2 * w) {
-                        const int mid = min(lo + w, n), hi = min(lo + 2 * w, n);
-                        int i = lo, j = mid, k = lo;
-                        while (i < mid && j < hi) T[k++] = A[j].x < A[i].x ? A[j++] : A[i++];
-                        while (i < mid) T[k++] = A[i++];
-                        while (j < hi) T[k++] = A[j++];
-                    }
-                    int3* t = A;
-                    A = T;
-                    T = t;
-                }
-                if (A != L)
-                    for (int a = 0; a < n; ++a) L[a] = A[a];
-            }
-            n4[sub] = walk_row(
-                n, mask, aa_width, cx.x, cx.y,
-                [&](int i, int32_t& x0, int32_t& x1, int32_t& cc) {
-                    x0 = L[i].x;
-                    x1 = L[i].y;
-                    cc = L[i].z;
-                },
-                [&](int q, int32_t s0, int32_t e0) {
-                    L[q].x = s0;
-                    L[q].y = e0;
-                },
-                nonterm);
-        }
         const uint32_t need = 4u * static_cast<uint32_t>(n4[0] + n4[1] + n4[2] + n4[3]);
         const uint32_t gi = group_off[p] + static_cast<uint32_t>(g - (P.y0 >> 2));
         const uint32_t o0 = need ? atomicAdd(&ctr->cell_cursor, need) : 0u;
