@@ -1138,6 +1138,33 @@ __host__ __device__ __forceinline__ int sweep_cells(const int (&n)[4], Bound bou
     return nc;
 }
 
+// The same cells from one list of the pixel row's n boundaries in column order,
+// 2 x (AA column) + (1: a span end). A boundary at column c changes its own
+// pixel by 4 - (c mod 4) columns and every later one by 4, so the pixel of a
+// run of boundaries has 4 x (depth before them) + the sum of their changes.
+template <typename Get, typename Put>
+__host__ __device__ __forceinline__ int sweep_sorted(int n, Get get, Put put) {
+    int depth = 0, nc = 0, cov = 0;
+    int32_t px = -1;  // the pixel being summed
+    auto emit = [&](int32_t x0, int32_t len, int32_t c) {
+        put(nc++, static_cast<uint32_t>(x0) | (static_cast<uint32_t>(len - 1) << 14) | (static_cast<uint32_t>(c - 1) << 28));
+    };
+    for (int i = 0; i < n; ++i) {
+        const int32_t b = get(i), col = b >> 1, q = col >> 2;
+        if (q != px) {
+            if (cov > 0) emit(px, 1, cov);
+            if (depth > 0 && q > px + 1) emit(px + 1, q - px - 1, 4 * depth);
+            px = q;
+            cov = 4 * depth;
+        }
+        const int32_t s = (b & 1) ? -1 : 1;
+        depth += s;
+        cov += s * (4 - (col & 3));
+    }
+    if (cov > 0) emit(px, 1, cov);
+    return nc;
+}
+
 // Merged Intersect lists of up to 32 consecutive AA rows of one path, one
 // row per lane, in shared memory: entry k of lane l at [k * LS + l].
 //
@@ -1192,31 +1219,29 @@ __device__ __forceinline__ int gather_row(const PathInfo& P, int32_t lo, int32_t
       uint32_t gm = __ballot_sync(0xffffffffu, g_hit);
       while (gm) {
         uint32_t mine[GS];
+        Edge e[GS];
+        bool hit[GS];
+        // The next GS groups' edges in flight together.
 #pragma unroll
         for (int s = 0; s < GS; ++s) {
-            mine[s] = 0;
-            // The next group with an edge on [lo, hi] goes to slot s.
-            while (gm) {
-                const uint32_t eb = (gb + static_cast<uint32_t>(__ffs(gm) - 1)) << 5;
-                gm &= gm - 1;
-                const uint32_t j = eb + lane;
-                Edge e;
-                bool hit = false;
-                if (j >= P.e_begin && j < P.e_end) {
-                    e = edges[j];
-                    hit = !(e.flags & EF_EMPTY) && e.row0 <= hi && e.row1 >= lo;
-                }
-                if (!__any_sync(0xffffffffu, hit)) continue;
-                uint32_t rows_of_edge = 0;
-                if (hit) {
-                    const int q = 32 * s + lane;
-                    sedge[q] = e;
-                    const int32_t ra = max(e.row0, lo) - lo, rb = min(e.row1, hi) - lo;
-                    rows_of_edge = (0xffffffffu >> (31 - rb)) & (0xffffffffu << ra);
-                }
-                mine[s] = warp_transpose32(rows_of_edge, lane);
-                break;
+            hit[s] = false;
+            if (!gm) continue;
+            const uint32_t j = ((gb + static_cast<uint32_t>(__ffs(gm) - 1)) << 5) + lane;
+            gm &= gm - 1;
+            if (j >= P.e_begin && j < P.e_end) {
+                e[s] = edges[j];
+                hit[s] = true;
             }
+        }
+#pragma unroll
+        for (int s = 0; s < GS; ++s) {
+            uint32_t rows_of_edge = 0;
+            if (hit[s] && !(e[s].flags & EF_EMPTY) && e[s].row0 <= hi && e[s].row1 >= lo) {
+                sedge[32 * s + lane] = e[s];
+                const int32_t ra = max(e[s].row0, lo) - lo, rb = min(e[s].row1, hi) - lo;
+                rows_of_edge = (0xffffffffu >> (31 - rb)) & (0xffffffffu << ra);
+            }
+            mine[s] = __any_sync(0xffffffffu, rows_of_edge != 0) ? warp_transpose32(rows_of_edge, lane) : 0u;
             if (!valid) mine[s] = 0;
         }
         __syncwarp();
@@ -1364,18 +1389,53 @@ __global__ void __launch_bounds__(WARPS * 32) k_rows(
         const int2 cx = path_clip ? make_int2(path_clip[p].x, path_clip[p].y) : make_int2(0, aa_width);
         if (valid && !overflow)
             ns = sort_and_walk<32>(n, mask, aa_width, cx.x, cx.y, sx0[w], sx1[w], scn[w], lane, nonterm);
-        // ---- one pixel row per 4 lanes: merge the sub-rows' spans into cells
-        sns[w][lane] = (valid && !overflow) ? ns : 0;
+        // ---- one pixel row per 4 lanes: the sub-rows' span boundaries in one
+        // sorted list, each lane placing its own: a boundary's place is its
+        // index in its list plus the boundaries before it in the other three
+        // (lists of lower lanes first among equal columns), found by stepping
+        // through them. A row has at most (n + 1) / 2 <= KCAP / 2 spans, so the
+        // list of a pixel row fits in its part of scn, which is free by now.
+        if (!valid || overflow) ns = 0;
+        sns[w][lane] = ns;
         const uint32_t ovf_lanes = __ballot_sync(0xffffffffu, overflow);
         __syncwarp();
         const bool leader = (lane & 3) == 0 && r <= P.y1;  // this pixel row has an AA row in [y0, y1]
         const bool g_ovf = ((ovf_lanes >> (lane & ~3)) & 0xFu) != 0;
-        int n4[4] = {0, 0, 0, 0};
+        int32_t* merged = &scn[w][(lane >> 2) * (4 * KCAP)];
+        if (!g_ovf) {
+            const int quad = lane & ~3;
+            int at[3], n3[3];  // per other list: the next boundary to compare, and their number
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                at[k] = 0;
+                n3[k] = 2 * sns[w][quad + ((lane + 1 + k) & 3)];
+            }
+            auto bound = [&](int i, int l) {
+                return (i & 1) ? sx1[w][(i >> 1) * 32 + l] : sx0[w][(i >> 1) * 32 + l];
+            };
+            for (int i = 0; i < 2 * ns; ++i) {
+                const int32_t c = bound(i, lane);
+                int place = i;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const int l = quad + ((lane + 1 + k) & 3);
+                    while (at[k] < n3[k]) {
+                        const int32_t o = bound(at[k], l);
+                        if (o > c || (o == c && l > lane)) break;
+                        ++at[k];
+                    }
+                    place += at[k];
+                }
+                merged[place] = 2 * c + (i & 1);
+            }
+        }
+        __syncwarp();
         uint32_t need = 0;
+        int n_bounds = 0;
         if (leader && !g_ovf) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) n4[k] = sns[w][lane + k];
-            need = 4u * static_cast<uint32_t>(n4[0] + n4[1] + n4[2] + n4[3]);  // 2 cells per span boundary
+            for (int k = 0; k < 4; ++k) n_bounds += 2 * sns[w][lane + k];
+            need = 2u * static_cast<uint32_t>(n_bounds);  // 2 cells per span boundary
         }
         uint32_t incl = need;
         for (int o = 1; o < 32; o <<= 1) {
@@ -1398,12 +1458,8 @@ __global__ void __launch_bounds__(WARPS * 32) k_rows(
                 group_idx[gi] = make_uint2(0u, 0u);
             } else if (fits) {
                 const uint32_t o0 = base + incl - need;
-                const int nc = sweep_cells(
-                    n4,
-                    [&](int k, int i, bool end) {
-                        return end ? sx1[w][i * 32 + lane + k] : sx0[w][i * 32 + lane + k];
-                    },
-                    [&](int q, uint32_t cell) { cells[o0 + q] = cell; });
+                const int nc = sweep_sorted(
+                    n_bounds, [&](int i) { return merged[i]; }, [&](int q, uint32_t cell) { cells[o0 + q] = cell; });
                 group_idx[gi] = make_uint2(o0, static_cast<uint32_t>(nc));
             } else {
                 group_idx[gi] = make_uint2(0u, 0u);
