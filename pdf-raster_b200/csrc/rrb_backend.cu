@@ -182,6 +182,13 @@ int grid_for(rrb_ctx* c, uint64_t n, int threads, int per_sm = 8) {
     return static_cast<int>(std::max<uint64_t>(1, std::min(need, cap)));
 }
 
+// Blocks of 256 for a warp per path, and up to per_sm blocks per SM where paths
+// are few: long ones take a block each (for_long_paths).
+int grid_for_paths(rrb_ctx* c, uint64_t n_paths, int per_sm) {
+    const uint64_t most = static_cast<uint64_t>(c->sm_count) * per_sm;
+    return std::max(grid_for(c, n_paths * 32, 256, per_sm), static_cast<int>(std::min(n_paths, most)));
+}
+
 // Exclusive scan of n u32 at d_in into d_out[0..n] (d_out[n] = total).
 int scan_u32(rrb_ctx* c, const uint32_t* d_in, uint32_t* d_out, uint32_t n) {
     uint32_t* bs = as<uint32_t>(c->s_block);
@@ -632,7 +639,7 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
                                                              B->has_hairline ? as<uint8_t>(B->rule) : nullptr,
                                                              kLongWalk);
     c->launches += 1;
-    k_walk_long<<<grid_for(c, n_paths * 32, 256, 16), 256, 0, c->stream>>>(
+    k_walk_long<<<grid_for_paths(c, n_paths, 16), WALK_THREADS, 0, c->stream>>>(
         as<double>(B->pts), as<uint8_t>(B->flags), as<uint64_t>(B->off), NP, as<double>(B->mtx),
         as<uint2>(c->s_slots), as<uint32_t>(c->s_path_pieces), B->has_hairline ? as<uint8_t>(B->rule) : nullptr,
         kLongWalk);
@@ -647,7 +654,7 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
     if (pclip && (rc = ensure(c, c->s_clip_lo, std::max<uint64_t>(1, n_pieces) * sizeof(uint32_t)))) return rc;
     uint32_t* clip_lo = pclip ? as<uint32_t>(c->s_clip_lo) : nullptr;
     if ((rc = ensure(c, c->s_edge_off, (n_pieces + 1) * sizeof(uint32_t)))) return rc;
-    k_compact_pieces<<<grid_for(c, n_paths * 32, 256, 16), 256, 0, c->stream>>>(
+    k_compact_pieces<<<grid_for_paths(c, n_paths, 16), 256, 0, c->stream>>>(
         as<uint64_t>(B->off), as<uint32_t>(c->s_path_pieces), NP, as<uint32_t>(B->page), as<uint32_t>(B->ph),
         as<uint2>(c->s_slots), as<uint2>(c->s_pieces), as<uint32_t>(c->s_clip), pclip, clip_lo);
     c->launches += 1;
@@ -700,7 +707,7 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
     stage_end(c, 3);
     const int chunk_rows = 32;
     stage(c, 4);
-    k_path_bbox<<<grid_for(c, n_paths * 32, 256), 256, 0, c->stream>>>(
+    k_path_bbox<<<grid_for_paths(c, n_paths, 8), 256, 0, c->stream>>>(
         as<uint32_t>(c->s_path_pieces), as<uint32_t>(c->s_edge_off), as<Edge>(c->s_edges), NP, as<uint8_t>(B->rule),
         as<uint8_t>(B->gray), as<uint8_t>(B->alpha), as<uint32_t>(B->page), as<uint32_t>(B->pw),
         as<uint32_t>(B->ph), rowmap, as<PathInfo>(c->s_info), as<uint32_t>(c->s_rows), as<uint32_t>(c->s_chunks),

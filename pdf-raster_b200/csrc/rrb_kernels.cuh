@@ -94,6 +94,27 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
     return m;
 }
 
+// f(p), by whole blocks, for the paths that is_long picks: a block looks at up
+// to 32 paths at a time (a lane of its first warp each), so that finding none
+// costs a page of 150,000 paths a few loads per block, and at fewer where there
+// are blocks enough (the picked paths of a group come one after another).
+template <typename IsLong, typename F>
+__device__ __forceinline__ void for_long_paths(uint32_t n_paths, const IsLong& is_long, const F& f) {
+    __shared__ uint32_t picked;
+    const uint32_t group = min(32u, (n_paths + gridDim.x - 1) / gridDim.x);
+    for (uint32_t base = blockIdx.x * group; base < n_paths; base += gridDim.x * group) {
+        if (threadIdx.x < 32) {
+            const uint32_t p = base + threadIdx.x;
+            const uint32_t m = __ballot_sync(0xffffffffu, threadIdx.x < group && p < n_paths && is_long(p));
+            if (threadIdx.x == 0) picked = m;
+        }
+        __syncthreads();
+        uint32_t m = picked;
+        __syncthreads();
+        for (; m; m &= m - 1) f(base + __ffs(m) - 1);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // XPath::new walk, one thread per path. Pieces are written at the path's
 // point slots [off, off+n); unused slots get PK_NONE. Point indices are global.
@@ -145,11 +166,14 @@ __global__ void k_walk(const double* __restrict__ pts, const uint8_t* __restrict
     }
 }
 
-// The same walk for paths of at least long_min points, one warp per path.
-// A serial walk of a long path (stroke outlines have thousands of points)
-// keeps one lane busy while its warp's other paths are done, and its lanes
-// diverge at every subpath end. Here each point's part in the walk is read
-// from its neighbours' flags, which is exact when the path is well formed:
+// The same walk for paths of at least long_min points, one warp per path, or
+// one block per path of at least WALK_BLOCK points. A serial walk of a long
+// path (stroke outlines have thousands of points) keeps one lane busy while its
+// warp's other paths are done, and its lanes diverge at every subpath end; a
+// warp takes a microsecond per 32 points of one path (latency), which left the
+// 7,000-point outlines of a stroke page's curves to finish alone: walk and
+// compaction 1.08 ms, by blocks 0.41. Here each point's part in the walk is read from its
+// neighbours' flags, which is exact when the path is well formed:
 // it starts with FIRST; CURVE points come in pairs after a non-CURVE point
 // and before a non-CURVE end point; no FIRST point is a control or end point;
 // no two consecutive points are FIRST; and a point after which the walk
@@ -161,20 +185,162 @@ __global__ void k_walk(const double* __restrict__ pts, const uint8_t* __restrict
 //   when it has LAST (the end point of a curve is never tested for LAST,
 //   xpath.rs:210-234);
 // and the closing test of a walk-subpath runs at each break and at the last
-// point, against the latest start. The warp scans 32 points at a time for
-// the latest start and the piece slots. A path that is not well formed is
-// walked serially by lane 0.
-__global__ void k_walk_long(const double* __restrict__ pts, const uint8_t* __restrict__ flags,
-                            const uint64_t* __restrict__ path_pt_off, uint32_t n_paths,
-                            const double* __restrict__ mtx, uint2* __restrict__ pieces,
-                            uint32_t* __restrict__ path_pieces, const uint8_t* __restrict__ rule,
-                            uint32_t long_min) {
+// point, against the latest start. The warp or block scans as many points as
+// it has threads at a time for the latest start and the piece slots. A path
+// that is not well formed is walked serially by one thread.
+constexpr uint32_t WALK_BLOCK = 1024;
+constexpr int WALK_THREADS = 256;
+
+struct WalkFlags {
+    const uint8_t* F;
+    int64_t n;
+    __device__ __forceinline__ uint32_t at(int64_t i) const { return (i >= 0 && i < n) ? F[i] : 0u; }
+    // Point i's share of the well-formedness of the path.
+    __device__ __forceinline__ bool good(int64_t i) const {
+        const uint32_t f0 = at(i), fm1 = at(i - 1), fm2 = at(i - 2), fp1 = at(i + 1), fp2 = at(i + 2);
+        const bool curve = f0 & PF_CURVE, pc = fm1 & PF_CURVE;
+        const bool ctrl1 = curve && !pc, ctrl2 = curve && pc, endpt = !curve && pc;
+        const bool lin = !curve && !endpt;
+        const bool prev_lin = i >= 1 && !pc && !(fm2 & PF_CURVE);
+        const bool start = (f0 & PF_FIRST) && (i == 0 || (prev_lin && (fm1 & PF_LAST)));
+        if (i == 0 && !(f0 & PF_FIRST)) return false;
+        if ((f0 & PF_FIRST) && (curve || endpt)) return false;
+        if (ctrl1 && !(i >= 1 && i + 2 < n && (fp1 & PF_CURVE) && !(fp2 & PF_CURVE))) return false;
+        if (ctrl2 && !(i >= 2 && !(fm2 & PF_CURVE))) return false;
+        if ((f0 & PF_FIRST) && (fm1 & PF_FIRST) && i >= 1) return false;
+        return !(lin && !start && (f0 & PF_LAST) && i + 1 < n && !(fp1 & PF_FIRST));
+    }
+    // Its part in the walk of a well-formed path.
+    __device__ __forceinline__ void part(int64_t i, bool& start, bool& piece, bool& is_curve, bool& close_ev) const {
+        const uint32_t f0 = at(i), fm1 = at(i - 1), fm2 = at(i - 2);
+        const bool curve = f0 & PF_CURVE, pc = fm1 & PF_CURVE;
+        const bool lin = !curve && !pc;
+        const bool prev_lin = i >= 1 && !pc && !(fm2 & PF_CURVE);
+        start = (f0 & PF_FIRST) && (i == 0 || (prev_lin && (fm1 & PF_LAST)));
+        is_curve = curve && !pc;
+        piece = is_curve || (lin && !start);
+        close_ev = (lin && !start && (f0 & PF_LAST)) || i == n - 1;
+    }
+};
+
+// Whether the walk closes a subpath from point a back to its start b.
+__device__ __forceinline__ bool walk_closes(const double* pts, const double* m, uint32_t a, uint32_t b) {
+    double sx, sy, cx, cy;
+    transform(m, pts[2 * b], pts[2 * b + 1], sx, sy);
+    transform(m, pts[2 * a], pts[2 * a + 1], cx, cy);
+    return fabs(dsub(cx, sx)) > 1e-10 || fabs(dsub(cy, sy)) > 1e-10;
+}
+
+// Serial walk of a path (the k_walk loop); returns its piece count.
+__device__ __noinline__ uint32_t walk_serial(const double* pts, const double* m, const uint8_t* F, uint32_t off,
+                                             uint32_t n, uint2* pieces) {
+    uint32_t slot = off, i = 0;
+    while (i < n) {
+        if (F[i] & PF_FIRST) {
+            uint32_t sp = i, cur = i;
+            ++i;
+            while (i < n) {
+                const uint8_t f = F[i];
+                if (f & PF_CURVE) {
+                    if (i + 2 >= n) break;
+                    pieces[slot++] = make_uint2(off + cur, (PK_CURVE << 30) | (off + i));
+                    cur = i + 2;
+                    i += 3;
+                } else {
+                    pieces[slot++] = make_uint2(off + cur, (PK_LINE << 30) | (off + i));
+                    cur = i;
+                    ++i;
+                    if (f & PF_LAST) break;
+                }
+            }
+            if (walk_closes(pts, m, off + cur, off + sp))
+                pieces[slot++] = make_uint2(off + cur, (PK_CLOSE << 30) | (off + sp));
+        } else {
+            ++i;
+        }
+    }
+    return slot - off;
+}
+
+__global__ void __launch_bounds__(WALK_THREADS) k_walk_long(
+    const double* __restrict__ pts, const uint8_t* __restrict__ flags, const uint64_t* __restrict__ path_pt_off,
+    uint32_t n_paths, const double* __restrict__ mtx, uint2* __restrict__ pieces, uint32_t* __restrict__ path_pieces,
+    const uint8_t* __restrict__ rule, uint32_t long_min) {
     __shared__ double m[6];
+    __shared__ int32_t warp_start[WALK_THREADS / 32];
+    __shared__ uint32_t warp_cnt[WALK_THREADS / 32];
     if (threadIdx.x < 6) m[threadIdx.x] = mtx[threadIdx.x];
     __syncthreads();
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < n_paths; p += warps) {
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // 32 points from b on by a warp: each lane's inclusive latest start and the
+    // slots of its piece and closing piece, given the start and slot before them.
+    auto step = [&](const WalkFlags& W, uint32_t off, int64_t i, auto&& scan) {
+        bool piece = false, is_curve = false, close_ev = false, start = false;
+        if (i < W.n) W.part(i, start, piece, is_curve, close_ev);
+        int32_t sp = start ? static_cast<int32_t>(i) : -1;  // latest start at or before the point
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t t = __shfl_up_sync(0xffffffffu, sp, o);
+            if (static_cast<int>(lane) >= o) sp = max(sp, t);
+        }
+        scan.starts(sp);
+        const bool close = close_ev && sp >= 0 &&
+                           walk_closes(pts, m, off + static_cast<uint32_t>(i), off + static_cast<uint32_t>(sp));
+        const uint32_t cnt = (piece ? 1u : 0u) + (close ? 1u : 0u);
+        uint32_t incl = cnt;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (static_cast<int>(lane) >= o) incl += t;
+        }
+        uint32_t at = scan.slots(incl) + incl - cnt;
+        if (piece)
+            pieces[at++] = make_uint2(off + static_cast<uint32_t>(i - 1),
+                                      ((is_curve ? PK_CURVE : PK_LINE) << 30) | (off + static_cast<uint32_t>(i)));
+        if (close)
+            pieces[at] = make_uint2(off + static_cast<uint32_t>(i), (PK_CLOSE << 30) | (off + static_cast<uint32_t>(sp)));
+    };
+    struct WarpScan {  // the steps of one warp, in order
+        int32_t last_start;
+        uint32_t slot;
+        __device__ __forceinline__ void starts(int32_t& sp) {
+            sp = max(sp, last_start);
+            last_start = __shfl_sync(0xffffffffu, sp, 31);
+        }
+        __device__ __forceinline__ uint32_t slots(uint32_t incl) {
+            const uint32_t at = slot;
+            slot += __shfl_sync(0xffffffffu, incl, 31);
+            return at;
+        }
+    };
+    struct BlockScan {  // the block's warps side by side
+        int32_t last_start;
+        uint32_t slot, lane, w;
+        int32_t* ws;
+        uint32_t* wc;
+        __device__ __forceinline__ void starts(int32_t& sp) {
+            if (lane == 31) ws[w] = sp;
+            __syncthreads();
+            int32_t before = last_start;
+#pragma unroll
+            for (int k = 0; k < WALK_THREADS / 32; ++k) {
+                before = max(before, k < static_cast<int>(w) ? ws[k] : -1);
+                last_start = max(last_start, ws[k]);
+            }
+            sp = max(sp, before);
+        }
+        __device__ __forceinline__ uint32_t slots(uint32_t incl) {
+            if (lane == 31) wc[w] = incl;
+            __syncthreads();
+            uint32_t at = slot;
+#pragma unroll
+            for (int k = 0; k < WALK_THREADS / 32; ++k) {
+                at += k < static_cast<int>(w) ? wc[k] : 0u;
+                slot += wc[k];
+            }
+            return at;
+        }
+    };
+    const uint32_t warps = gridDim.x * (WALK_THREADS / 32);
+    for (uint32_t p = blockIdx.x * (WALK_THREADS / 32) + w; p < n_paths; p += warps) {
         const uint32_t off = static_cast<uint32_t>(path_pt_off[p]);
         const uint32_t n = static_cast<uint32_t>(path_pt_off[p + 1]) - off;
         if (n < long_min) continue;
@@ -182,115 +348,37 @@ __global__ void k_walk_long(const double* __restrict__ pts, const uint8_t* __res
             if (lane == 0) path_pieces[p] = 0;
             continue;
         }
-        const uint8_t* F = flags + off;
-        auto fl = [&](int64_t i) -> uint32_t { return (i >= 0 && i < static_cast<int64_t>(n)) ? F[i] : 0u; };
-        // Well-formedness, 32 points at a time.
+        if (n >= WALK_BLOCK) continue;  // by a block, below
+        const WalkFlags W{flags + off, static_cast<int64_t>(n)};
         bool ok = true;
-        for (uint32_t b = 0; b < n && ok; b += 32) {
-            const int64_t i = static_cast<int64_t>(b) + lane;
-            bool good = true;
-            if (i < static_cast<int64_t>(n)) {
-                const uint32_t f0 = fl(i), fm1 = fl(i - 1), fm2 = fl(i - 2), fp1 = fl(i + 1), fp2 = fl(i + 2);
-                const bool curve = f0 & PF_CURVE, pc = fm1 & PF_CURVE;
-                const bool ctrl1 = curve && !pc, ctrl2 = curve && pc, endpt = !curve && pc;
-                const bool lin = !curve && !endpt;
-                const bool prev_lin = i >= 1 && !pc && !(fm2 & PF_CURVE);
-                const bool start = (f0 & PF_FIRST) && (i == 0 || (prev_lin && (fm1 & PF_LAST)));
-                if (i == 0 && !(f0 & PF_FIRST)) good = false;
-                if ((f0 & PF_FIRST) && (curve || endpt)) good = false;
-                if (ctrl1 && !(i >= 1 && i + 2 < static_cast<int64_t>(n) && (fp1 & PF_CURVE) && !(fp2 & PF_CURVE)))
-                    good = false;
-                if (ctrl2 && !(i >= 2 && !(fm2 & PF_CURVE))) good = false;
-                if ((f0 & PF_FIRST) && (fm1 & PF_FIRST) && i >= 1) good = false;
-                if (lin && !start && (f0 & PF_LAST) && i + 1 < static_cast<int64_t>(n) && !(fp1 & PF_FIRST))
-                    good = false;
-            }
-            ok = __all_sync(0xffffffffu, good);
-        }
-        if (!ok) {
-            // Serial walk of a path that is not well formed (the k_walk loop).
-            if (lane == 0) {
-                uint32_t slot = off, i = 0;
-                while (i < n) {
-                    if (F[i] & PF_FIRST) {
-                        uint32_t sp = i, cur = i;
-                        ++i;
-                        while (i < n) {
-                            const uint8_t f = F[i];
-                            if (f & PF_CURVE) {
-                                if (i + 2 >= n) break;
-                                pieces[slot++] = make_uint2(off + cur, (PK_CURVE << 30) | (off + i));
-                                cur = i + 2;
-                                i += 3;
-                            } else {
-                                pieces[slot++] = make_uint2(off + cur, (PK_LINE << 30) | (off + i));
-                                cur = i;
-                                ++i;
-                                if (f & PF_LAST) break;
-                            }
-                        }
-                        double sx, sy, cx, cy;
-                        transform(m, pts[2 * (off + sp)], pts[2 * (off + sp) + 1], sx, sy);
-                        transform(m, pts[2 * (off + cur)], pts[2 * (off + cur) + 1], cx, cy);
-                        if (fabs(dsub(cx, sx)) > 1e-10 || fabs(dsub(cy, sy)) > 1e-10)
-                            pieces[slot++] = make_uint2(off + cur, (PK_CLOSE << 30) | (off + sp));
-                    } else {
-                        ++i;
-                    }
-                }
-                path_pieces[p] = slot - off;
-            }
+        for (uint32_t i = lane; i < n; i += 32) ok &= W.good(i);
+        if (!__all_sync(0xffffffffu, ok)) {
+            if (lane == 0) path_pieces[p] = walk_serial(pts, m, W.F, off, n, pieces);
             continue;
         }
-        uint32_t slot_base = off;
-        int64_t last_start = -1;
-        for (uint32_t b = 0; b < n; b += 32) {
-            const int64_t i = static_cast<int64_t>(b) + lane;
-            const bool valid = i < static_cast<int64_t>(n);
-            bool piece = false, is_curve = false, close_ev = false, start = false;
-            if (valid) {
-                const uint32_t f0 = fl(i), fm1 = fl(i - 1), fm2 = fl(i - 2);
-                const bool curve = f0 & PF_CURVE, pc = fm1 & PF_CURVE;
-                const bool ctrl1 = curve && !pc, endpt = !curve && pc;
-                const bool lin = !curve && !endpt;
-                const bool prev_lin = i >= 1 && !pc && !(fm2 & PF_CURVE);
-                start = (f0 & PF_FIRST) && (i == 0 || (prev_lin && (fm1 & PF_LAST)));
-                is_curve = ctrl1;
-                piece = ctrl1 || (lin && !start);
-                const bool brk = lin && !start && (f0 & PF_LAST);
-                close_ev = brk || (i == static_cast<int64_t>(n) - 1);
-            }
-            // The latest start at or before each point.
-            int64_t sp = start ? i : -1;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int64_t t = __shfl_up_sync(0xffffffffu, sp, o);
-                if (static_cast<int>(lane) >= o) sp = max(sp, t);
-            }
-            sp = max(sp, last_start);
-            bool close = false;
-            if (close_ev && sp >= 0) {
-                double sx, sy, cx, cy;
-                transform(m, pts[2 * (off + sp)], pts[2 * (off + sp) + 1], sx, sy);
-                transform(m, pts[2 * (off + i)], pts[2 * (off + i) + 1], cx, cy);
-                close = fabs(dsub(cx, sx)) > 1e-10 || fabs(dsub(cy, sy)) > 1e-10;
-            }
-            const uint32_t cnt = (piece ? 1u : 0u) + (close ? 1u : 0u);
-            uint32_t incl = cnt;
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-                if (static_cast<int>(lane) >= o) incl += t;
-            }
-            uint32_t at = slot_base + incl - cnt;
-            if (piece)
-                pieces[at++] = make_uint2(off + static_cast<uint32_t>(i - 1),
-                                          ((is_curve ? PK_CURVE : PK_LINE) << 30) | (off + static_cast<uint32_t>(i)));
-            if (close)
-                pieces[at] = make_uint2(off + static_cast<uint32_t>(i), (PK_CLOSE << 30) | (off + static_cast<uint32_t>(sp)));
-            slot_base += __shfl_sync(0xffffffffu, incl, 31);
-            last_start = __shfl_sync(0xffffffffu, sp, 31);
-        }
-        if (lane == 0) path_pieces[p] = slot_base - off;
+        WarpScan scan{-1, off};
+        for (uint32_t b = 0; b < n; b += 32) step(W, off, static_cast<int64_t>(b) + lane, scan);
+        if (lane == 0) path_pieces[p] = scan.slot - off;
     }
+    auto is_long = [&](uint32_t p) {
+        return path_pt_off[p + 1] - path_pt_off[p] >= max(long_min, WALK_BLOCK) && !(rule && rule[p] == RULE_HAIRLINE);
+    };
+    for_long_paths(n_paths, is_long, [&](uint32_t p) {
+        const uint32_t off = static_cast<uint32_t>(path_pt_off[p]);
+        const uint32_t n = static_cast<uint32_t>(path_pt_off[p + 1]) - off;
+        const WalkFlags W{flags + off, static_cast<int64_t>(n)};
+        bool ok = true;
+        for (uint32_t i = threadIdx.x; i < n; i += WALK_THREADS) ok &= W.good(i);
+        if (!__syncthreads_and(ok)) {
+            if (threadIdx.x == 0) path_pieces[p] = walk_serial(pts, m, W.F, off, n, pieces);
+            return;
+        }
+        BlockScan scan{-1, off, lane, w, warp_start, warp_cnt};
+        // Each step's second barrier orders its first pair of reads before the next step's writes.
+        for (uint32_t b = 0; b < n; b += WALK_THREADS) step(W, off, static_cast<int64_t>(b) + threadIdx.x, scan);
+        if (threadIdx.x == 0) path_pieces[p] = scan.slot - off;
+        __syncthreads();
+    });
 }
 
 // Pack each path's pieces (the first path_pieces[p] slots of its point range)
@@ -301,11 +389,9 @@ __global__ void k_compact_pieces(const uint64_t* __restrict__ path_pt_off, const
                                  const uint32_t* __restrict__ page_h, const uint2* __restrict__ slots,
                                  uint2* __restrict__ pieces, uint32_t* __restrict__ piece_clip,
                                  const int4* __restrict__ path_clip, uint32_t* __restrict__ piece_clip_lo) {
-    // One warp per path: its lanes copy the pieces (long stroke outlines have
-    // thousands) in coalesced strides.
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < n_paths; p += warps) {
+    // One warp per path copies its pieces in coalesced strides, one block those
+    // of at least WALK_BLOCK points (long stroke outlines).
+    auto copy = [&](uint32_t p, uint32_t first, uint32_t stride) {
         const uint32_t src = static_cast<uint32_t>(path_pt_off[p]);
         const uint32_t dst = piece_off[p], n = piece_off[p + 1] - dst;
         uint32_t clip_hi = 4u * page_h[path_page[p]] - 1u, clip_lo = 0;
@@ -314,12 +400,17 @@ __global__ void k_compact_pieces(const uint64_t* __restrict__ path_pt_off, const
             clip_lo = static_cast<uint32_t>(cl.z);
             clip_hi = static_cast<uint32_t>(cl.w);
         }
-        for (uint32_t k = lane; k < n; k += 32) {
+        for (uint32_t k = first; k < n; k += stride) {
             pieces[dst + k] = slots[src + k];
             piece_clip[dst + k] = clip_hi;
             if (piece_clip_lo) piece_clip_lo[dst + k] = clip_lo;
         }
-    }
+    };
+    auto is_long = [&](uint32_t p) { return path_pt_off[p + 1] - path_pt_off[p] >= WALK_BLOCK; };
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < n_paths; p += warps)
+        if (!is_long(p)) copy(p, threadIdx.x & 31, 32);
+    for_long_paths(n_paths, is_long, [&](uint32_t p) { copy(p, threadIdx.x, blockDim.x); });
 }
 
 __device__ __forceinline__ void load_tpt(const double* pts, const double* m, uint32_t i, double& x, double& y) {
@@ -636,6 +727,8 @@ __global__ void k_scan_down(const uint32_t* __restrict__ in, uint32_t* __restric
 // read under the as-shipped row map only) gives per path the pixel rows the
 // shipped driver loop visits when they come from another path's AA range.
 // ---------------------------------------------------------------------------
+constexpr uint32_t BBOX_BLOCK = 1024;
+
 __global__ void RRB_BBOX_BOUNDS k_path_bbox(const uint32_t* __restrict__ piece_off, const uint32_t* __restrict__ edge_off,
                             const Edge* __restrict__ edges, uint32_t n_paths, const uint8_t* __restrict__ rule,
                             const uint8_t* __restrict__ gray, const uint8_t* __restrict__ alpha,
@@ -645,23 +738,25 @@ __global__ void RRB_BBOX_BOUNDS k_path_bbox(const uint32_t* __restrict__ piece_o
                             int chunk_rows, BatchCounters* __restrict__ ctr, int32_t* __restrict__ gmin,
                             int32_t* __restrict__ gmax, const int4* __restrict__ path_clip,
                             const int2* __restrict__ path_visit) {
-    int lane = threadIdx.x & 31;
-    uint32_t warp_g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t warp_g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     // The batch's sums, kept by each warp's lanes and added up once per block.
     // Two atomics per path on two addresses (1.4 ns each, one after another)
     // bound the kernel before: 150,000 glyphs (55 M edge records, 1.76 GB)
     // 0.75 -> 0.31 ms, 5.7 TB/s; warp reductions in one instruction each took a
-    // page of 40 long paths from 90 to 71 us (a warp per path: latency).
+    // page of 40 long paths from 90 to 71 us, a block for each of them to 18 us.
     unsigned long long sum_raw = 0, sum_rows = 0;
-    for (uint32_t p = warp_g; p < n_paths; p += nwarps) {
-        uint32_t eb = edge_off[piece_off[p]], ee = edge_off[piece_off[p + 1]];
-        int32_t y0 = INT32_MAX, y1 = INT32_MIN, xl = INT32_MAX, xh = INT32_MIN;
-        unsigned long long raw = 0;
-        bool axis_only = true;
+    struct Bounds {
+        int32_t y0, y1, xl, xh;
+        int32_t axis_only;
+    };
+    // A warp's bounds of the 128-edge steps at first, first + stride, ... of [eb, ee).
+    auto scan = [&](uint32_t eb, uint32_t ee, uint32_t first, uint32_t stride) {
+        Bounds B{INT32_MAX, INT32_MIN, INT32_MAX, INT32_MIN, 1};
         // Aligned groups of 32 edges: one group per iteration, its row range
         // merged into gmin/gmax (atomically: a group can straddle two paths).
-        for (uint32_t base4 = eb & ~31u; base4 < ee; base4 += 128) {
+        for (uint32_t base4 = (eb & ~31u) + first; base4 < ee; base4 += stride) {
           // Four groups' loads in flight before any is reduced.
           Edge e4[4];
 #pragma unroll
@@ -680,31 +775,34 @@ __global__ void RRB_BBOX_BOUNDS k_path_bbox(const uint32_t* __restrict__ piece_o
                 if (!(e.flags & EF_EMPTY)) {
                     int32_t lo, hi;
                     edge_xrange(e, lo, hi);
-                    raw += static_cast<unsigned long long>(e.row1 - e.row0 + 1);
-                    y0 = min(y0, e.row0);
-                    y1 = max(y1, e.row1);
-                    xl = min(xl, lo);
-                    xh = max(xh, hi);
+                    sum_raw += static_cast<unsigned long long>(e.row1 - e.row0 + 1);
+                    B.y0 = min(B.y0, e.row0);
+                    B.y1 = max(B.y1, e.row1);
+                    B.xl = min(B.xl, lo);
+                    B.xh = max(B.xh, hi);
                     g0 = e.row0;
                     g1 = e.row1;
                 }
             }
             g0 = __reduce_min_sync(0xffffffffu, g0);
             g1 = __reduce_max_sync(0xffffffffu, g1);
-            axis_only &= (e4[u].flags & EF_EMPTY) || (e4[u].flags & EF_KIND_MASK) != EK_SLOPED;
+            B.axis_only &= (e4[u].flags & EF_EMPTY) || (e4[u].flags & EF_KIND_MASK) != EK_SLOPED;
             if (lane == 0 && g0 <= g1) {
                 atomicMin(&gmin[base >> 5], g0);
                 atomicMax(&gmax[base >> 5], g1);
             }
           }
         }
-        y0 = __reduce_min_sync(0xffffffffu, y0);
-        y1 = __reduce_max_sync(0xffffffffu, y1);
-        xl = __reduce_min_sync(0xffffffffu, xl);
-        xh = __reduce_max_sync(0xffffffffu, xh);
-        axis_only = __all_sync(0xffffffffu, axis_only);
-        sum_raw += raw;
-        if (lane == 0) {
+        B.y0 = __reduce_min_sync(0xffffffffu, B.y0);
+        B.y1 = __reduce_max_sync(0xffffffffu, B.y1);
+        B.xl = __reduce_min_sync(0xffffffffu, B.xl);
+        B.xh = __reduce_max_sync(0xffffffffu, B.xh);
+        B.axis_only = __all_sync(0xffffffffu, B.axis_only);
+        return B;
+    };
+    auto finish = [&](uint32_t p, uint32_t eb, uint32_t ee, const Bounds& B) {
+            const int32_t y0 = B.y0, y1 = B.y1, xl = B.xl, xh = B.xh;
+            const bool axis_only = B.axis_only != 0;
             if (y0 <= y1) sum_rows += static_cast<unsigned long long>(y1 - y0 + 1);
             uint32_t pg = path_page[p];
             int32_t W = static_cast<int32_t>(page_w[pg]), H = static_cast<int32_t>(page_h[pg]);
@@ -765,8 +863,34 @@ __global__ void RRB_BBOX_BOUNDS k_path_bbox(const uint32_t* __restrict__ piece_o
             // Rectilinear paths skip the row stage: k_recti builds their row runs.
             path_groups[p] = recti ? 0u : groups;
             path_chunks[p] = recti ? 0u : (rows + chunk_rows - 1) / chunk_rows;
-        }
+    };
+    for (uint32_t p = warp_g; p < n_paths; p += nwarps) {
+        const uint32_t eb = edge_off[piece_off[p]], ee = edge_off[piece_off[p + 1]];
+        if (ee - eb >= BBOX_BLOCK) continue;  // by a block, below
+        const Bounds B = scan(eb, ee, 0, 128);
+        if (lane == 0) finish(p, eb, ee, B);
     }
+    // Paths of BBOX_BLOCK edges and more: the warps of a block side by side.
+    __shared__ Bounds part[32];
+    auto is_long = [&](uint32_t p) { return edge_off[piece_off[p + 1]] - edge_off[piece_off[p]] >= BBOX_BLOCK; };
+    for_long_paths(n_paths, is_long, [&](uint32_t p) {
+        const uint32_t eb = edge_off[piece_off[p]], ee = edge_off[piece_off[p + 1]];
+        const Bounds mine = scan(eb, ee, 128 * w, 4 * blockDim.x);
+        if (lane == 0) part[w] = mine;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            Bounds B = mine;
+            for (uint32_t k = 1; k < blockDim.x / 32; ++k) {
+                B.y0 = min(B.y0, part[k].y0);
+                B.y1 = max(B.y1, part[k].y1);
+                B.xl = min(B.xl, part[k].xl);
+                B.xh = max(B.xh, part[k].xh);
+                B.axis_only &= part[k].axis_only;
+            }
+            finish(p, eb, ee, B);
+        }
+        __syncthreads();
+    });
     __shared__ unsigned long long block_raw, block_rows;
     if (threadIdx.x == 0) block_raw = block_rows = 0;
     __syncthreads();
