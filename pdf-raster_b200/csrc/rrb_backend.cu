@@ -661,15 +661,16 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
     stage_end(c, 0);
     RRB_CUDA(c, cudaGetLastError());
     stage(c, 1);
-    // Curves of more than CURVE_BIG segments: listed here, counted by a warp each.
+    // Curves of more than big_min segments: listed here, counted by a warp each.
     if ((rc = ensure(c, c->s_big, std::max<uint64_t>(1, n_pieces) * sizeof(uint32_t)))) return rc;
     // Lane counts of the first lane_cap big curves: the write pass places each
     // lane's leaves from them instead of counting again (later curves recount).
     const uint32_t lane_cap = static_cast<uint32_t>(std::min<uint64_t>(n_pieces, kLaneCountCurves));
     if ((rc = ensure(c, c->s_lanes, std::max<uint64_t>(1, lane_cap) * CURVE_LANES))) return rc;
+    const int big_min = n_pieces <= CURVE_FEW_PIECES ? 1 : CURVE_BIG;
     k_seg_count<true><<<grid_for(c, n_pieces, 128, 32), 128, 0, c->stream>>>(
         as<double>(B->pts), as<uint2>(c->s_pieces), NPC, as<double>(B->mtx), flat_sq, as<uint32_t>(c->s_edge_off),
-        as<uint32_t>(c->s_big), as<BatchCounters>(c->s_ctr));
+        as<uint32_t>(c->s_big), as<BatchCounters>(c->s_ctr), big_min);
     k_seg_count_big<<<c->sm_count * 16, 128, 0, c->stream>>>(as<double>(B->pts), as<uint2>(c->s_pieces),
                                                             as<double>(B->mtx), flat_sq, as<uint32_t>(c->s_big),
                                                             as<BatchCounters>(c->s_ctr), as<uint32_t>(c->s_edge_off),
@@ -698,7 +699,7 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
     stage(c, 3);
     k_seg_write<true><<<grid_for(c, n_pieces, 128, 32), 128, 0, c->stream>>>(
         as<double>(B->pts), as<uint2>(c->s_pieces), NPC, as<double>(B->mtx), flat_sq, as<uint32_t>(c->s_edge_off),
-        static_cast<uint32_t>(n_edges), as<Edge>(c->s_edges), as<uint32_t>(c->s_clip), clip_lo);
+        static_cast<uint32_t>(n_edges), as<Edge>(c->s_edges), as<uint32_t>(c->s_clip), clip_lo, big_min);
     k_seg_write_big<<<c->sm_count * 16, 128, 0, c->stream>>>(
         as<double>(B->pts), as<uint2>(c->s_pieces), as<double>(B->mtx), flat_sq, as<uint32_t>(c->s_big),
         as<BatchCounters>(c->s_ctr), as<uint32_t>(c->s_edge_off), static_cast<uint32_t>(n_edges),

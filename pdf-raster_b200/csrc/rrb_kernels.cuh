@@ -418,10 +418,18 @@ __device__ __forceinline__ void load_tpt(const double* pts, const double* m, uin
 }
 
 // Curves of more than this many segments are flattened by a warp each
-// (k_seg_count_big / k_seg_write_big): thread-per-curve work is that long.
-constexpr int CURVE_BIG = 32;
+// (k_seg_count_big / k_seg_write_big): thread-per-curve work is that long, a
+// chain of FP64 latencies, and as uneven as the curves of a warp. 16 against 32:
+// 9 mixed pages count 1.40 -> 1.26 ms, write 2.64 -> 2.38; 8 loses on text
+// (curves of 5 segments: count 40 -> 46 us).
+constexpr int CURVE_BIG = 16;
+// With few pieces the chip is idle and the longest chain is the stage's time:
+// every curve of more than one segment goes to a warp (1,382 pieces: count 37
+// -> 24 us, write 91 -> 50; 33,000: 54 -> 41, 131 -> 86; 73,000: 91 -> 64, 174
+// -> 135; but 294,000 pieces of text 40 -> 143, 95 -> 228).
+constexpr uint32_t CURVE_FEW_PIECES = 128u << 10;
 
-// Segments per piece slot. SPLIT: a curve with more than CURVE_BIG segments
+// Segments per piece slot. SPLIT: a curve with more than big_min segments
 // is counted 0 here and appended to big_list (big-curve count in
 // ctr->big_curves) for k_seg_count_big.
 // Register budgets (CTAs per SM the compiler must fit; 0: its own choice)
@@ -446,7 +454,8 @@ constexpr int CURVE_BIG = 32;
 template <bool SPLIT>
 __global__ void RRB_SEG_BOUNDS k_seg_count(const double* __restrict__ pts, const uint2* __restrict__ pieces, uint32_t n_slots,
                             const double* __restrict__ mtx, double flat_sq, uint32_t* __restrict__ counts,
-                            uint32_t* __restrict__ big_list, BatchCounters* __restrict__ ctr) {
+                            uint32_t* __restrict__ big_list, BatchCounters* __restrict__ ctr,
+                            int big_min = CURVE_BIG) {
     __shared__ double m[6];
     if (threadIdx.x < 6) m[threadIdx.x] = mtx[threadIdx.x];
     __syncthreads();
@@ -468,8 +477,8 @@ __global__ void RRB_SEG_BOUNDS k_seg_count(const double* __restrict__ pts, const
             load_tpt(pts, m, i + 1, x2, y2);
             load_tpt(pts, m, i + 2, x3, y3);
             if (SPLIT) {
-                c = static_cast<uint32_t>(flatten_count_capped(x0, y0, x1, y1, x2, y2, x3, y3, flat_sq, CURVE_BIG));
-                big = c > static_cast<uint32_t>(CURVE_BIG);
+                c = static_cast<uint32_t>(flatten_count_capped(x0, y0, x1, y1, x2, y2, x3, y3, flat_sq, big_min));
+                big = c > static_cast<uint32_t>(big_min);
                 if (big) c = 0;
             } else {
                 c = flatten_curve(x0, y0, x1, y1, x2, y2, x3, y3, flat_sq, [](double, double) {});
@@ -544,12 +553,13 @@ __global__ void RRB_BIG_CURVE_BOUNDS k_seg_count_big(const double* __restrict__ 
 }
 
 // Edge records per piece slot, at edge_off[slot]. SPLIT: curves with more
-// than CURVE_BIG segments are left to k_seg_write_big.
+// than big_min segments are left to k_seg_write_big.
 template <bool SPLIT>
 __global__ void RRB_SEG_BOUNDS k_seg_write(const double* __restrict__ pts, const uint2* __restrict__ pieces, uint32_t n_slots,
                             const double* __restrict__ mtx, double flat_sq, const uint32_t* __restrict__ edge_off,
                             uint32_t edge_cap, Edge* __restrict__ edges,
-                            const uint32_t* __restrict__ slot_clip_hi, const uint32_t* __restrict__ slot_clip_lo) {
+                            const uint32_t* __restrict__ slot_clip_hi, const uint32_t* __restrict__ slot_clip_lo,
+                            int big_min = CURVE_BIG) {
     __shared__ double m[6];
     if (threadIdx.x < 6) m[threadIdx.x] = mtx[threadIdx.x];
     __syncthreads();
@@ -558,7 +568,7 @@ __global__ void RRB_SEG_BOUNDS k_seg_write(const double* __restrict__ pts, const
         uint32_t kind = pc.y >> 30;
         if (kind == PK_NONE) continue;
         uint32_t base = edge_off[s];
-        if (SPLIT && kind == PK_CURVE && edge_off[s + 1] - base > static_cast<uint32_t>(CURVE_BIG)) continue;
+        if (SPLIT && kind == PK_CURVE && edge_off[s + 1] - base > static_cast<uint32_t>(big_min)) continue;
         int32_t chi = static_cast<int32_t>(slot_clip_hi[s]);
         const int32_t clo = slot_clip_lo ? static_cast<int32_t>(slot_clip_lo[s]) : 0;
         uint32_t j = pc.y & 0x3fffffffu;
