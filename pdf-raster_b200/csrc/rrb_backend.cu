@@ -51,6 +51,8 @@ constexpr int KCAP_WIDE = 16;   // the same for the 4-warp row-stage shapes
 // stages warps x groups x 32 edges (512, 256, 256, 1024, 128).
 constexpr int kRowShapes = 5;
 constexpr uint64_t kLaneCountCurves = 1ull << 22;  // big curves whose lane counts are kept (128 MiB)
+constexpr uint32_t kLongWalk = 64;    // path points from which a warp walks a path
+constexpr uint64_t kFewPaths = 4096;  // paths up to which warps walk them all (one launch)
 constexpr int SUPER = 256;      // supertile edge in pixels (a multiple of every tile shape)
 
 }  // namespace
@@ -112,6 +114,7 @@ struct rrb_ctx {
     // by its trials (0: none yet, 64x16), the default of batches uploaded per
     // call on this context until another batch settles or the tuning changes.
     uint32_t settled_tw = 0, settled_th = 0;
+    cudaEvent_t size_ev[3] = {nullptr, nullptr, nullptr};  // counters read back behind the launches (send_counters)
     cudaEvent_t trial_ev[2] = {nullptr, nullptr};  // timing of a resident batch's trial render
 };
 
@@ -189,22 +192,39 @@ int grid_for_paths(rrb_ctx* c, uint64_t n_paths, int per_sm) {
     return std::max(grid_for(c, n_paths * 32, 256, per_sm), static_cast<int>(std::min(n_paths, most)));
 }
 
-// Exclusive scan of n u32 at d_in into d_out[0..n] (d_out[n] = total).
-int scan_u32(rrb_ctx* c, const uint32_t* d_in, uint32_t* d_out, uint32_t n) {
-    uint32_t* bs = as<uint32_t>(c->s_block);
-    if (n == 0) {
-        RRB_CUDA(c, cudaMemsetAsync(d_out, 0, sizeof(uint32_t), c->stream));
+// Exclusive scan of job.in[0..n) into job.out[0..n] (out[n] = the total, which
+// also goes where job.total says). bound: an upper bound of the count, which
+// is job.n or, on the device, *job.n_ptr.
+int scan_u32(rrb_ctx* c, const ScanJob& job, uint64_t bound) {
+    if (bound <= SCAN_SMALL) {
+        k_scan_jobs<<<1, 1024, 0, c->stream>>>(ScanJobs{{job, job}});
+        c->launches += 1;
+        RRB_CUDA(c, cudaGetLastError());
         return RRB_OK;
     }
+    uint32_t* bs = as<uint32_t>(c->s_block);
+    const uint32_t n = static_cast<uint32_t>(bound);
     uint32_t nb = std::min<uint32_t>(SCAN_MAX_BLOCKS, std::max<uint32_t>(1, (n + 4095) / 4096));
     uint32_t per = (n + nb - 1) / nb;
     nb = (n + per - 1) / per;
-    k_scan_reduce<<<nb, SCAN_THREADS, 0, c->stream>>>(d_in, n, per, bs);
-    k_scan_blocks<<<1, 1024, 0, c->stream>>>(bs, nb);
-    k_scan_down<<<nb, SCAN_THREADS, 0, c->stream>>>(d_in, d_out, n, per, bs);
+    k_scan_reduce<<<nb, SCAN_THREADS, 0, c->stream>>>(job.in, job.n, per, bs, job.n_ptr);
+    k_scan_blocks<<<1, 1024, 0, c->stream>>>(bs, nb, job.total);
+    k_scan_down<<<nb, SCAN_THREADS, 0, c->stream>>>(job.in, job.out, job.n, per, bs, job.n_ptr);
     c->launches += 3;
     RRB_CUDA(c, cudaGetLastError());
     return RRB_OK;
+}
+
+// Two scans whose inputs are ready together.
+int scan_u32_pair(rrb_ctx* c, const ScanJob& a, const ScanJob& b) {
+    if (std::max(a.n, b.n) <= SCAN_SMALL) {
+        k_scan_jobs<<<2, 1024, 0, c->stream>>>(ScanJobs{{a, b}});
+        c->launches += 1;
+        RRB_CUDA(c, cudaGetLastError());
+        return RRB_OK;
+    }
+    const int rc = scan_u32(c, a, a.n);
+    return rc ? rc : scan_u32(c, b, b.n);
 }
 
 template <typename T>
@@ -212,6 +232,26 @@ int upload(rrb_ctx* c, Scratch& s, const T* src, size_t count) {
     int rc = ensure(c, s, count * sizeof(T));
     if (rc) return rc;
     if (count) RRB_CUDA(c, cudaMemcpyAsync(s.p, src, count * sizeof(T), cudaMemcpyHostToDevice, c->stream));
+    return RRB_OK;
+}
+
+// A batch's counters as they stand at this point of the stream, into slot k of
+// the page-locked readback area; wait_counters waits for them.
+constexpr size_t kCounterSlot = 128;  // 32-bit words from one slot to the next, the first at word 128
+static_assert(sizeof(BatchCounters) <= kCounterSlot * 4, "a slot holds the counters");
+
+int send_counters(rrb_ctx* c, int k) {
+    if (!c->size_ev[k]) RRB_CUDA(c, cudaEventCreateWithFlags(&c->size_ev[k], cudaEventDisableTiming));
+    RRB_CUDA(c, cudaMemcpyAsync(c->h_read + (k + 1) * kCounterSlot, c->s_ctr.p, sizeof(BatchCounters),
+                                cudaMemcpyDeviceToHost, c->stream));
+    RRB_CUDA(c, cudaEventRecord(c->size_ev[k], c->stream));
+    return RRB_OK;
+}
+
+int wait_counters(rrb_ctx* c, int k, BatchCounters& out) {
+    ++c->host_syncs;
+    RRB_CUDA(c, cudaEventSynchronize(c->size_ev[k]));
+    std::memcpy(&out, c->h_read + (k + 1) * kCounterSlot, sizeof out);
     return RRB_OK;
 }
 
@@ -246,6 +286,15 @@ void preload_trial_kernels() {
     RRB_PRELOAD_COMP(64, 16);
     RRB_PRELOAD_COMP(128, 16);
     RRB_PRELOAD_COMP(128, 32);
+    // The row stage's shared memory exceeds the 48 KB that need no asking.
+    auto rows_smem = [](auto kernel, size_t bytes) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+    };
+    rows_smem(k_rows<KCAP, ROWS_WARPS>, rows_smem_bytes<KCAP, ROWS_WARPS>());
+    rows_smem(k_rows<KCAP_WIDE, 4>, rows_smem_bytes<KCAP_WIDE, 4>());
+    rows_smem(k_rows<KCAP, ROWS_WARPS, 1>, rows_smem_bytes<KCAP, ROWS_WARPS, 1>());
+    rows_smem(k_rows<8, 16>, rows_smem_bytes<8, 16>());
+    rows_smem(k_rows<KCAP_WIDE, 4, 1>, rows_smem_bytes<KCAP_WIDE, 4, 1>());
     RRB_PRELOAD(k_rows<KCAP, ROWS_WARPS>);
     RRB_PRELOAD(k_rows<KCAP_WIDE, 4>);
     RRB_PRELOAD(k_rows<KCAP, ROWS_WARPS, 1>);
@@ -581,14 +630,51 @@ int batch_upload(rrb_ctx* c, const rrb_path_batch_params* h, rrb_batch* B, const
     return RRB_OK;
 }
 
+// A batch uploaded per call with up to this many points is first launched whole, without waiting for a size: each stage reads its counts on the device,
+// the buffers that a count sizes are taken as the context's earlier renders left
+// them, and a count beyond its buffer stops every later stage before it touches
+// anything (BatchCounters::err; the pages are only written by the last). The
+// sizes come back behind the launches and are checked as they arrive; where one
+// did not fit, the batch is rendered again with the sizes read back between the
+// stages, which grows the buffers. Six waits of 10-15 us with the device idle
+// become none, calls of one glyph 304 -> 198 us, of 40 paths 475 -> 370, of 900
+// paths under clips 812 -> 692. Larger batches gain nothing by it.
+constexpr uint64_t kFreePoints = 2ull << 20;
+
 // The pipeline over a device-resident batch into the device page arena.
 // ws: the wave's cached sizes (see WaveSizes), or nullptr. When they match,
 // every stage is launched without waiting on the stream, and the counters
 // are copied into the page-locked slot c->h_waves[slot] for the caller to
 // read after its one wait (c->deferred is set); otherwise the sizes are read
-// back between the stages and, if ws is given, stored there.
+// back between the stages (free: behind them, see kFreePoints) and, if ws is
+// given, stored there. free: *retry is set, and nothing rendered, where a size
+// did not fit.
+int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int rowmap, WaveSizes* ws, uint32_t slot,
+                 bool free, bool* retry);
+
 int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int rowmap,
                      WaveSizes* ws = nullptr, uint32_t slot = 0) {
+    // Batches uploaded per call only: a kept batch pays for its waits once, and
+    // launches exactly what its sizes ask for from then on. The buffers sized by
+    // counts must exist (some render has sized them).
+    const bool free = B == c->tmp_batch && B->n_pts <= kFreePoints && c->s_edges.p && c->s_groups.p && c->s_row_idx.p && c->s_ovf.p &&
+                      c->s_ovf2.p && c->s_spans.p && c->s_super_list.p && c->s_runs.p && c->s_chunk_path.p &&
+                      c->s_chunk_live.p;
+    bool retry = false;
+    const bool pages_pending = c->wait_pages_up;
+    int rc = run_pipeline(c, B, arena, arena_len, rowmap, ws, slot, free, &retry);
+    // Its buffers per point are bounds: without room for them, by size too.
+    if (free && rc == RRB_ERR_OUT_OF_MEMORY) {
+        RRB_CUDA(c, cudaStreamSynchronize(c->stream));
+        retry = true;
+    }
+    if (!retry) return rc;
+    c->wait_pages_up = pages_pending;
+    return run_pipeline(c, B, arena, arena_len, rowmap, ws, slot, false, nullptr);
+}
+
+int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int rowmap, WaveSizes* ws, uint32_t slot,
+                 bool free, bool* retry) {
     c->launches = 0;
     c->host_syncs = 0;
     c->deferred = false;
@@ -609,6 +695,8 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
     set_tiles(B->geom_h, tw, th, tiles);
     if (tiles >= (1ull << 31)) return set_err(c, RRB_ERR_INVARIANT, "too many tiles");
     const bool cached = ws && ws->matches(tw, th, B->row_shape, rowmap) && slot < c->h_waves_cap;
+    if (cached) free = false;
+    const bool sized = !cached && !free;  // sizes are read back between the stages
     const uint64_t n_paths = B->n_paths, n_pts = B->n_pts, supers = B->supers;
     const uint32_t n_pages = B->n_pages;
     const uint32_t NP = static_cast<uint32_t>(n_paths);
@@ -630,24 +718,31 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
     if ((rc = ensure(c, c->s_ctr, sizeof(BatchCounters)))) return rc;
     RRB_CUDA(c, cudaMemsetAsync(c->s_ctr.p, 0, sizeof(BatchCounters), c->stream));
     stage(c, 0);
-    // Paths of up to kLongWalk points: a thread each; longer ones: a warp each.
-    constexpr uint32_t kLongWalk = 64;
-    k_walk<<<grid_for(c, n_paths, 128, 32), 128, 0, c->stream>>>(as<double>(B->pts), as<uint8_t>(B->flags),
-                                                             as<uint64_t>(B->off), NP, as<double>(B->mtx),
-                                                             as<uint32_t>(B->page), as<uint32_t>(B->ph),
-                                                             as<uint2>(c->s_slots), as<uint32_t>(c->s_path_pieces),
-                                                             B->has_hairline ? as<uint8_t>(B->rule) : nullptr,
-                                                             kLongWalk);
-    c->launches += 1;
+    BatchCounters* ctr = as<BatchCounters>(c->s_ctr);
+    // Paths of up to kLongWalk points: a thread each; longer ones: a warp each
+    // (every path where there are few of them), or a block.
+    const uint32_t long_walk = n_paths <= kFewPaths ? 0 : kLongWalk;
+    if (long_walk) {
+        k_walk<<<grid_for(c, n_paths, 128, 32), 128, 0, c->stream>>>(
+            as<double>(B->pts), as<uint8_t>(B->flags), as<uint64_t>(B->off), NP, as<double>(B->mtx),
+            as<uint32_t>(B->page), as<uint32_t>(B->ph), as<uint2>(c->s_slots), as<uint32_t>(c->s_path_pieces),
+            B->has_hairline ? as<uint8_t>(B->rule) : nullptr, long_walk);
+        c->launches += 1;
+    }
     k_walk_long<<<grid_for_paths(c, n_paths, 16), WALK_THREADS, 0, c->stream>>>(
         as<double>(B->pts), as<uint8_t>(B->flags), as<uint64_t>(B->off), NP, as<double>(B->mtx),
         as<uint2>(c->s_slots), as<uint32_t>(c->s_path_pieces), B->has_hairline ? as<uint8_t>(B->rule) : nullptr,
-        kLongWalk);
+        long_walk);
     c->launches += 1;
     RRB_CUDA(c, cudaGetLastError());
-    if ((rc = scan_u32(c, as<uint32_t>(c->s_path_pieces), as<uint32_t>(c->s_path_pieces), NP))) return rc;
-    if (!cached && (rc = read_back(c, as<uint32_t>(c->s_path_pieces) + NP, sizeof(uint32_t)))) return rc;
-    const uint64_t n_pieces = cached ? ws->n_pieces : c->h_read[0];
+    constexpr uint32_t kNoCap = 0xFFFFFFFFu;
+    uint32_t* path_pieces = as<uint32_t>(c->s_path_pieces);
+    if ((rc = scan_u32(c, ScanJob{path_pieces, path_pieces, NP, nullptr, ScanTotal{&ctr->n_pieces, kNoCap, 0, nullptr, ctr}},
+                       NP)))
+        return rc;
+    if (sized && (rc = read_back(c, path_pieces + NP, sizeof(uint32_t)))) return rc;
+    // A path has at most one piece per point.
+    const uint64_t n_pieces = cached ? ws->n_pieces : free ? n_pts : c->h_read[0];
     const uint32_t NPC = static_cast<uint32_t>(n_pieces);
     if ((rc = ensure(c, c->s_pieces, std::max<uint64_t>(1, n_pieces) * sizeof(uint2)))) return rc;
     if ((rc = ensure(c, c->s_clip, std::max<uint64_t>(1, n_pieces) * sizeof(uint32_t)))) return rc;
@@ -679,27 +774,35 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
     stage_end(c, 1);
     RRB_CUDA(c, cudaGetLastError());
     stage(c, 2);
-    if ((rc = scan_u32(c, as<uint32_t>(c->s_edge_off), as<uint32_t>(c->s_edge_off), NPC))) return rc;
+    // What a count may reach (free: what its buffers hold; the kernels behind
+    // stop at the error otherwise).
+    auto cap32 = [](uint64_t v) { return static_cast<uint32_t>(std::min<uint64_t>(v, 0xFFFFFF00ull)); };
+    const uint64_t free_edges = std::min<uint64_t>(c->s_edges.cap / sizeof(Edge), (c->s_groups.cap / 8 - 2) * 32);
+    uint32_t* edge_off = as<uint32_t>(c->s_edge_off);
+    if ((rc = scan_u32(c, ScanJob{edge_off, edge_off, 0, &ctr->n_pieces,
+                                  ScanTotal{&ctr->n_edges, free ? cap32(free_edges) : kNoCap, ERR_EDGE_CAP, nullptr, ctr}},
+                       n_pieces)))
+        return rc;
     stage_end(c, 2);
-    if (!cached && (rc = read_back(c, as<uint32_t>(c->s_edge_off) + NPC, sizeof(uint32_t)))) return rc;
-    const uint64_t n_edges = cached ? ws->n_edges : c->h_read[0];
+    if (free && (rc = send_counters(c, 0))) return rc;
+    if (sized && (rc = read_back(c, &ctr->n_edges, sizeof(uint32_t)))) return rc;
+    const uint64_t n_edges = cached ? ws->n_edges : free ? cap32(free_edges) : c->h_read[0];
     // ---- stage 2: edges, path boxes, row/chunk offsets, supertile bins
     if ((rc = ensure(c, c->s_edges, std::max<uint64_t>(1, n_edges) * sizeof(Edge)))) return rc;
     if ((rc = ensure(c, c->s_info, n_paths * sizeof(PathInfo)))) return rc;
     if ((rc = ensure(c, c->s_rows, (n_paths + 1) * sizeof(uint32_t)))) return rc;
     if ((rc = ensure(c, c->s_chunks, (n_paths + 1) * sizeof(uint32_t)))) return rc;
     if ((rc = ensure(c, c->s_super_cnt, (supers + 1) * sizeof(uint32_t)))) return rc;
-    const uint64_t n_egroups = (n_edges + 31) / 32 + 1;
+    const uint64_t n_egroups = free ? c->s_groups.cap / 8 : (n_edges + 31) / 32 + 1;
     if ((rc = ensure(c, c->s_groups, n_egroups * 2 * sizeof(int32_t)))) return rc;
     int32_t* gmin = as<int32_t>(c->s_groups);
     int32_t* gmax = gmin + n_egroups;
-    // 0x7f7f7f7f / 0x80808080: beyond any AA row, so they act as +inf / -inf.
-    RRB_CUDA(c, cudaMemsetAsync(gmin, 0x7f, n_egroups * sizeof(int32_t), c->stream));
-    RRB_CUDA(c, cudaMemsetAsync(gmax, 0x80, n_egroups * sizeof(int32_t), c->stream));
+    k_init_groups<<<free ? grid_for(c, n_pts / 8, 256, 2) : grid_for(c, n_egroups, 256), 256, 0, c->stream>>>(gmin, gmax, ctr);
+    c->launches += 1;
     stage(c, 3);
     k_seg_write<true><<<grid_for(c, n_pieces, 128, 32), 128, 0, c->stream>>>(
         as<double>(B->pts), as<uint2>(c->s_pieces), NPC, as<double>(B->mtx), flat_sq, as<uint32_t>(c->s_edge_off),
-        static_cast<uint32_t>(n_edges), as<Edge>(c->s_edges), as<uint32_t>(c->s_clip), clip_lo, big_min);
+        static_cast<uint32_t>(n_edges), as<Edge>(c->s_edges), as<uint32_t>(c->s_clip), clip_lo, big_min, ctr);
     k_seg_write_big<<<c->sm_count * 16, 128, 0, c->stream>>>(
         as<double>(B->pts), as<uint2>(c->s_pieces), as<double>(B->mtx), flat_sq, as<uint32_t>(c->s_big),
         as<BatchCounters>(c->s_ctr), as<uint32_t>(c->s_edge_off), static_cast<uint32_t>(n_edges),
@@ -729,27 +832,46 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
     stage_end(c, 4);
     RRB_CUDA(c, cudaGetLastError());
     stage(c, 5);
-    if ((rc = scan_u32(c, as<uint32_t>(c->s_rows), as<uint32_t>(c->s_rows), NP))) return rc;
-    if ((rc = scan_u32(c, as<uint32_t>(c->s_chunks), as<uint32_t>(c->s_chunks), NP))) return rc;
+    // 32-bit offsets: refused where the paths' AA rows could have wrapped them
+    // (free: rendered again with sizes, which checks as it always has).
+    const uint64_t free_groups = std::min(std::min(c->s_row_idx.cap, c->s_ovf.cap), c->s_ovf2.cap) / sizeof(uint2);
+    const uint64_t free_chunks = std::min<uint64_t>(c->s_chunk_path.cap / sizeof(uint2), c->s_chunk_live.cap - 4);
+    const unsigned long long* rows_wide = free ? &ctr->aa_rows : nullptr;
+    uint32_t *path_rows = as<uint32_t>(c->s_rows), *path_chunks = as<uint32_t>(c->s_chunks);
+    if ((rc = scan_u32_pair(
+             c,
+             ScanJob{path_rows, path_rows, NP, nullptr,
+                     ScanTotal{&ctr->n_groups, free ? cap32(free_groups) : kNoCap, ERR_ROW_CAP, rows_wide, ctr}},
+             ScanJob{path_chunks, path_chunks, NP, nullptr,
+                     ScanTotal{&ctr->n_chunks, free ? cap32(free_chunks) : kNoCap, ERR_ROW_CAP, rows_wide, ctr}})))
+        return rc;
     stage_end(c, 5);
     const uint32_t NSUP = static_cast<uint32_t>(supers);
     stage(c, 6);
     k_super_bin<false><<<grid_for(c, supers * 32, 256), 256, 0, c->stream>>>(
         as<PathInfo>(c->s_info), as<PageGeom>(B->geom), n_pages, NSUP, SUPER, SUPER, as<uint32_t>(c->s_super_cnt),
-        nullptr, nullptr);
+        nullptr, nullptr, nullptr, ctr);
     c->launches += 1;
     stage_end(c, 6);
     RRB_CUDA(c, cudaGetLastError());
     stage(c, 7);
-    if ((rc = scan_u32(c, as<uint32_t>(c->s_super_cnt), as<uint32_t>(c->s_super_cnt), NSUP))) return rc;
     // Rectilinear paths: runs per path, then their offsets.
     k_recti<false><<<grid_for(c, n_paths, 128, 16), 128, 0, c->stream>>>(
         as<PathInfo>(c->s_info), NP, as<Edge>(c->s_edges), as<uint32_t>(B->pw), rowmap, as<uint32_t>(c->s_run_off),
-        nullptr, nullptr, nullptr, 0, as<BatchCounters>(c->s_ctr), pclip);
+        nullptr, nullptr, nullptr, 0, ctr, pclip);
     c->launches += 1;
     RRB_CUDA(c, cudaGetLastError());
-    if ((rc = scan_u32(c, as<uint32_t>(c->s_run_off), as<uint32_t>(c->s_run_off), NP))) return rc;
+    uint32_t *super_cnt = as<uint32_t>(c->s_super_cnt), *path_runs = as<uint32_t>(c->s_run_off);
+    if ((rc = scan_u32_pair(
+             c,
+             ScanJob{super_cnt, super_cnt, NSUP, nullptr,
+                     ScanTotal{&ctr->n_pairs, free ? cap32(c->s_super_list.cap / 4) : kNoCap, ERR_SUPER_CAP, nullptr, ctr}},
+             ScanJob{path_runs, path_runs, NP, nullptr,
+                     ScanTotal{&ctr->n_runs, free ? cap32(c->s_runs.cap / sizeof(int4)) : kNoCap, ERR_RUN_CAP,
+                               free ? &ctr->hl_rows : nullptr, ctr}})))
+        return rc;
     stage_end(c, 7);
+    if (free && (rc = send_counters(c, 1))) return rc;
     uint64_t n_groups, n_chunks, n_pairs, n_runs, raw_entries, hl_rows;
     if (cached) {
         n_groups = ws->n_groups;
@@ -758,50 +880,56 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
         n_runs = ws->n_runs;
         raw_entries = ws->raw_entries;
         hl_rows = ws->hl_rows;
+    } else if (free) {
+        n_groups = free_groups;
+        n_chunks = free_chunks;
+        n_pairs = c->s_super_list.cap / 4;
+        n_runs = c->s_runs.cap / sizeof(int4);
+        raw_entries = hl_rows = 0;
     } else {
-        RRB_CUDA(c, cudaMemcpyAsync(c->h_read + 0, as<uint32_t>(c->s_rows) + NP, 4, cudaMemcpyDeviceToHost,
-                                    c->stream));
-        RRB_CUDA(c, cudaMemcpyAsync(c->h_read + 1, as<uint32_t>(c->s_chunks) + NP, 4, cudaMemcpyDeviceToHost,
-                                    c->stream));
-        RRB_CUDA(c, cudaMemcpyAsync(c->h_read + 2, as<uint32_t>(c->s_super_cnt) + NSUP, 4, cudaMemcpyDeviceToHost,
-                                    c->stream));
-        RRB_CUDA(c, cudaMemcpyAsync(c->h_read + 4, &as<BatchCounters>(c->s_ctr)->raw_entries, 8,
-                                    cudaMemcpyDeviceToHost, c->stream));
-        RRB_CUDA(c, cudaMemcpyAsync(c->h_read + 6, as<uint32_t>(c->s_run_off) + NP, 4, cudaMemcpyDeviceToHost,
-                                    c->stream));
-        RRB_CUDA(c, cudaMemcpyAsync(c->h_read + 8, &as<BatchCounters>(c->s_ctr)->hl_rows, 8, cudaMemcpyDeviceToHost,
-                                    c->stream));
-        ++c->host_syncs;
-        RRB_CUDA(c, cudaStreamSynchronize(c->stream));
-        n_groups = c->h_read[0];
-        n_chunks = c->h_read[1];
-        n_pairs = c->h_read[2];
-        n_runs = c->h_read[6];
-        std::memcpy(&raw_entries, c->h_read + 4, 8);
-        std::memcpy(&hl_rows, c->h_read + 8, 8);
+        if ((rc = read_back(c, ctr, sizeof(BatchCounters)))) return rc;
+        BatchCounters hs;
+        std::memcpy(&hs, c->h_read, sizeof hs);
+        n_groups = hs.n_groups;
+        n_chunks = hs.n_chunks;
+        n_pairs = hs.n_pairs;
+        n_runs = hs.n_runs;
+        raw_entries = hs.raw_entries;
+        hl_rows = hs.hl_rows;
     }
     // The run offsets were scanned in 32 bits: refuse totals that could wrap.
-    if (hl_rows > 0x7FFFFFFFull || n_runs > 0x7FFFFFFFull)
+    if (!free && (hl_rows > 0x7FFFFFFFull || n_runs > 0x7FFFFFFFull))
         return set_err(c, RRB_ERR_POOL_EXHAUSTED, "batch needs more than 2^31 row runs");
     // ---- stage 3: rows -> coverage cells. An AA row with m merged entries
     // yields at most m/2 + 1 spans, and a pixel row at most 2 cells per span
     // boundary: cells <= 4 * spans <= 2 * raw entries + 4 * AA rows.
     const uint64_t aa_rows = 4 * n_groups;
     uint64_t cell_cap = 2 * raw_entries + 4 * aa_rows + hl_rows + 1024;
+    if (free) cell_cap = std::min<uint64_t>(c->s_spans.cap / sizeof(uint32_t), 0xFFFFFF00ull);
     if (cell_cap > 0xFFFFFF00ull) return set_err(c, RRB_ERR_POOL_EXHAUSTED, "batch needs more than 2^32 cells");
-    if (n_groups > 0x3FFFFFFFull) return set_err(c, RRB_ERR_POOL_EXHAUSTED, "batch needs more than 2^30 pixel rows");
-    if ((rc = ensure(c, c->s_row_idx, std::max<uint64_t>(1, n_groups) * sizeof(uint2)))) return rc;
-    if ((rc = ensure(c, c->s_spans, cell_cap * sizeof(uint32_t)))) return rc;
-    if ((rc = ensure(c, c->s_ovf, std::max<uint64_t>(1, n_groups) * sizeof(uint2)))) return rc;
-    if ((rc = ensure(c, c->s_super_list, std::max<uint64_t>(1, n_pairs) * sizeof(uint32_t)))) return rc;
-    if ((rc = ensure(c, c->s_runs, std::max<uint64_t>(1, n_runs) * sizeof(int4)))) return rc;
+    if (!free && n_groups > 0x3FFFFFFFull) return set_err(c, RRB_ERR_POOL_EXHAUSTED, "batch needs more than 2^30 pixel rows");
+    if (!free) {
+        if ((rc = ensure(c, c->s_row_idx, std::max<uint64_t>(1, n_groups) * sizeof(uint2)))) return rc;
+        if ((rc = ensure(c, c->s_spans, cell_cap * sizeof(uint32_t)))) return rc;
+        if ((rc = ensure(c, c->s_ovf, std::max<uint64_t>(1, n_groups) * sizeof(uint2)))) return rc;
+        if ((rc = ensure(c, c->s_ovf2, std::max<uint64_t>(1, n_groups) * sizeof(uint2)))) return rc;
+        if ((rc = ensure(c, c->s_super_list, std::max<uint64_t>(1, n_pairs) * sizeof(uint32_t)))) return rc;
+        if ((rc = ensure(c, c->s_runs, std::max<uint64_t>(1, n_runs) * sizeof(int4)))) return rc;
+        if ((rc = ensure(c, c->s_chunk_live, n_chunks + 8))) return rc;
+        if ((rc = ensure(c, c->s_chunk_path, std::max<uint64_t>(1, n_chunks) * sizeof(uint2)))) return rc;
+    }
+    // The most row chunks the paths can have, for the grids of free renders.
+    uint64_t most_chunks = n_chunks;
+    if (free) {
+        most_chunks = 0;
+        for (const PageGeom& G : B->geom_h) most_chunks += static_cast<uint64_t>(G.path_end - G.path_begin) * (G.h / 8 + 2);
+        most_chunks = std::min(most_chunks, n_chunks);
+    }
     if ((rc = ensure(c, c->s_tile_start, tiles * sizeof(uint32_t)))) return rc;
-    if ((rc = ensure(c, c->s_chunk_live, std::max<uint64_t>(1, n_chunks)))) return rc;
-    RRB_CUDA(c, cudaMemsetAsync(c->s_chunk_live.p, 0, std::max<uint64_t>(1, n_chunks), c->stream));
     stage(c, 8);
     k_super_bin<true><<<grid_for(c, supers * 32, 256), 256, 0, c->stream>>>(
         as<PathInfo>(c->s_info), as<PageGeom>(B->geom), n_pages, NSUP, SUPER, SUPER, nullptr,
-        as<uint32_t>(c->s_super_cnt), as<uint32_t>(c->s_super_list));
+        as<uint32_t>(c->s_super_cnt), as<uint32_t>(c->s_super_list), as<uint32_t>(c->s_chunk_live), ctr);
     c->launches += 1;
     if (n_runs) {  // before k_tile_start, which reads the solid boxes
         k_recti<true><<<grid_for(c, n_paths, 128, 16), 128, 0, c->stream>>>(
@@ -820,7 +948,6 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
     RRB_CUDA(c, cudaGetLastError());
     stage(c, 9);
     if (n_chunks) {
-        if ((rc = ensure(c, c->s_chunk_path, n_chunks * sizeof(uint2)))) return rc;
         k_chunk_paths<<<grid_for(c, n_paths * 32, 256), 256, 0, c->stream>>>(
             as<uint32_t>(c->s_chunks), NP, as<uint8_t>(c->s_chunk_live), as<uint2>(c->s_chunk_path),
             as<BatchCounters>(c->s_ctr));
@@ -830,9 +957,7 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
         // k_groups_mid: pages whose rows carry more crossings), 8 entries with
         // 16 warps, each with one or two edge groups staged per warp.
         auto rows = [&](auto kernel, int warps, size_t smem) -> int {
-            RRB_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(smem)));
-            kernel<<<grid_for(c, n_chunks * 32, warps * 32, 16), warps * 32, smem, c->stream>>>(
+            kernel<<<grid_for(c, most_chunks * 32, warps * 32, 16), warps * 32, smem, c->stream>>>(
                 as<PathInfo>(c->s_info), as<uint32_t>(c->s_chunks), as<uint32_t>(c->s_rows), as<Edge>(c->s_edges),
                 gmin, gmax, as<uint32_t>(B->pw), as<uint2>(c->s_row_idx), as<uint32_t>(c->s_spans),
                 static_cast<uint32_t>(cell_cap), as<uint2>(c->s_ovf), static_cast<uint32_t>(std::max<uint64_t>(1, n_groups)),
@@ -849,7 +974,7 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
         if (rc) return rc;
         c->launches += 1;
     }
-    if (B->has_hairline && hl_rows) {
+    if (B->has_hairline && (hl_rows || free)) {
         k_hl_write<<<grid_for(c, n_paths * 32, 256, 8), 256, 0, c->stream>>>(
             as<double>(B->pts), as<uint64_t>(B->off), as<uint8_t>(B->rule), as<double>(B->mtx),
             as<uint32_t>(B->page), as<uint32_t>(B->pw), as<uint32_t>(B->ph), hl_clip, NP, rowmap,
@@ -863,15 +988,15 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
     // sequential path for rows longer than its shared lists.
     BatchCounters hc;
     std::memset(&hc, 0, sizeof hc);
-    if (!cached) {
+    if (sized) {
         if ((rc = read_back(c, as<BatchCounters>(c->s_ctr), sizeof(BatchCounters)))) return rc;
         std::memcpy(&hc, c->h_read, sizeof hc);
     }
-    const uint32_t ovf_cap = static_cast<uint32_t>(std::max<uint64_t>(1, n_groups));
-    const uint64_t mid = cached ? ws->mid : std::min<uint64_t>(hc.ovf_count, n_groups);
+    const uint32_t ovf_cap = cap32(std::max<uint64_t>(1, n_groups));
+    // Free renders launch both overflow kernels: they find their row counts on the device.
+    uint64_t mid = cached ? ws->mid : free ? std::min<uint64_t>(8 * most_chunks, n_groups) : std::min<uint64_t>(hc.ovf_count, n_groups);
     uint64_t slow = 0, slow_need = 0;
     if (mid) {
-        if ((rc = ensure(c, c->s_ovf2, std::max<uint64_t>(1, n_groups) * sizeof(uint2)))) return rc;
         stage(c, 10);
         k_groups_mid<<<grid_for(c, mid * 32, MID_WARPS * 32, 16), MID_WARPS * 32, 0, c->stream>>>(
             as<PathInfo>(c->s_info), as<uint32_t>(c->s_rows), as<Edge>(c->s_edges), gmin, gmax,
@@ -879,15 +1004,15 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
             static_cast<uint32_t>(cell_cap), as<uint2>(c->s_ovf2), as<BatchCounters>(c->s_ctr), pclip);
         c->launches += 1;
         RRB_CUDA(c, cudaGetLastError());
-        if (!cached) {
+        if (sized) {
             if ((rc = read_back(c, as<BatchCounters>(c->s_ctr), sizeof(BatchCounters)))) return rc;
             std::memcpy(&hc, c->h_read, sizeof hc);
         }
-        slow = cached ? ws->slow : std::min<uint64_t>(hc.ovf2_count, n_groups);
-        if (slow && cached) {
-            // The scratch the last render settled on; the cursors are where the
-            // faster paths left them on the device.
-            slow_need = ws->slow_need;
+        slow = cached ? ws->slow : free ? mid : std::min<uint64_t>(hc.ovf2_count, n_groups);
+        if (slow && !sized) {
+            // The scratch the last render settled on (free: what there is); the
+            // cursors are where the faster paths left them on the device.
+            slow_need = cached ? ws->slow_need : 0;
             if ((rc = ensure(c, c->s_scratch, slow_need * sizeof(int3)))) return rc;
             k_groups_slow<<<grid_for(c, slow * 32, SLOW_WARPS * 32, 16), SLOW_WARPS * 32, 0, c->stream>>>(
                 as<PathInfo>(c->s_info), as<uint32_t>(c->s_rows), as<Edge>(c->s_edges), gmin, gmax,
@@ -964,16 +1089,39 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
         c->stats.host_syncs = c->host_syncs;
         return RRB_OK;
     }
-    if ((rc = read_back(c, as<BatchCounters>(c->s_ctr), sizeof(BatchCounters)))) return rc;
-    std::memcpy(&hc, c->h_read, sizeof hc);
+    if (free) {
+        // The sizes in the order they came; an error in one ends the render
+        // (the stages behind it have done nothing).
+        if ((rc = send_counters(c, 2))) return rc;
+        for (int k = 0; k < 3; ++k) {
+            if ((rc = wait_counters(c, k, hc))) return rc;
+            if (hc.err) {
+                RRB_CUDA(c, cudaEventSynchronize(c->size_ev[2]));  // before any buffer grows
+                *retry = true;
+                return RRB_OK;
+            }
+        }
+        n_groups = hc.n_groups;
+        n_chunks = hc.n_chunks;
+        n_pairs = hc.n_pairs;
+        n_runs = hc.n_runs;
+        raw_entries = hc.raw_entries;
+        hl_rows = hc.hl_rows;
+        mid = hc.ovf_count;
+        slow = hc.ovf2_count;
+        slow_need = hc.scratch_cursor;
+    } else {
+        if ((rc = read_back(c, as<BatchCounters>(c->s_ctr), sizeof(BatchCounters)))) return rc;
+        std::memcpy(&hc, c->h_read, sizeof hc);
+    }
     if (ws && !hc.err) {
         ws->valid = true;
         ws->tw = tw;
         ws->th = th;
         ws->row_shape = B->row_shape;
         ws->rowmap = rowmap;
-        ws->n_pieces = n_pieces;
-        ws->n_edges = n_edges;
+        ws->n_pieces = hc.n_pieces;
+        ws->n_edges = hc.n_edges;
         ws->n_groups = n_groups;
         ws->n_chunks = n_chunks;
         ws->n_pairs = n_pairs;
@@ -985,12 +1133,11 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
         ws->slow_need = slow_need;
     }
     c->stats.paths = n_paths;
-    c->stats.pieces = n_pieces;
-    c->stats.segments = n_edges;
+    c->stats.segments = hc.n_edges;
     c->stats.aa_rows = hc.aa_rows;
     c->stats.spans = hc.cell_cursor;
     c->stats.row_overflows = hc.ovf_count;
-    c->stats.pieces = n_pieces;
+    c->stats.pieces = hc.n_pieces;
     c->stats.tiles = tiles;
     c->stats.tile_pairs = n_pairs;
     c->stats.nonterminating_rows = hc.nonterminating;
@@ -1723,6 +1870,8 @@ int rrb_destroy(rrb_ctx* c) {
     for (Scratch* s : all) dev_free(c, s->p, s->cap);
     for (Scratch& s : c->s_fill) dev_free(c, s.p, s.cap);
     for (cudaEvent_t e : c->trial_ev)
+        if (e) cudaEventDestroy(e);
+    for (cudaEvent_t e : c->size_ev)
         if (e) cudaEventDestroy(e);
     if (c->tmp_batch) {
         free_batch_bufs(c, c->tmp_batch);

@@ -171,6 +171,7 @@ __global__ void k_hl_count(const double* __restrict__ pts, const uint64_t* __res
                            int rowmap, PathInfo* __restrict__ info, uint32_t* __restrict__ run_count,
                            BatchCounters* __restrict__ ctr) {
     __shared__ double m[6];
+    if (ctr->err) return;
     if (threadIdx.x < 6) m[threadIdx.x] = mtx[threadIdx.x];
     __syncthreads();
     unsigned long long total = 0;
@@ -228,6 +229,7 @@ __global__ void k_hl_write(const double* __restrict__ pts, const uint64_t* __res
                            PathInfo* __restrict__ info, int4* __restrict__ runs, uint32_t* __restrict__ cells,
                            uint32_t cell_cap, BatchCounters* __restrict__ ctr) {
     __shared__ double m[6];
+    if (ctr->err) return;
     if (threadIdx.x < 6) m[threadIdx.x] = mtx[threadIdx.x];
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31;

@@ -58,7 +58,7 @@ constexpr uint32_t RECTI_MAX_EDGES = 32;
 
 // Error / status word bits shared by all kernels of a batch.
 constexpr uint32_t ERR_EDGE_CAP = 1, ERR_ROW_CAP = 2, ERR_SPAN_CAP = 4, ERR_OVF_CAP = 8,
-                   ERR_SCRATCH_CAP = 16, ERR_SUPER_CAP = 32;
+                   ERR_SCRATCH_CAP = 16, ERR_SUPER_CAP = 32, ERR_RUN_CAP = 64;
 
 // Device counters of a batch.
 struct BatchCounters {
@@ -72,6 +72,9 @@ struct BatchCounters {
     uint32_t big_curves;   // curves flattened by a warp each (k_seg_count's big_list)
     uint32_t solid;        // paths whose solid box may hold a tile (k_recti): 0 = no tile has full layers
     uint32_t live_chunks;  // row chunks that some tile reads (k_chunk_paths)
+    // Sizes that the stages find (the scans' totals): the later stages read them
+    // here, so none of them has to be launched with one.
+    uint32_t n_pieces, n_edges, n_groups, n_chunks, n_pairs, n_runs;
     unsigned long long raw_entries;  // sum over edges of the rows they cover
     unsigned long long aa_rows;      // sum over paths of y1 - y0 + 1
     unsigned long long hl_rows;      // hairline segments: pixel rows drawn (one run and one cell each)
@@ -456,6 +459,7 @@ __global__ void RRB_SEG_BOUNDS k_seg_count(const double* __restrict__ pts, const
                             const double* __restrict__ mtx, double flat_sq, uint32_t* __restrict__ counts,
                             uint32_t* __restrict__ big_list, BatchCounters* __restrict__ ctr,
                             int big_min = CURVE_BIG) {
+    if (SPLIT) n_slots = ctr->n_pieces;
     __shared__ double m[6];
     if (threadIdx.x < 6) m[threadIdx.x] = mtx[threadIdx.x];
     __syncthreads();
@@ -559,7 +563,8 @@ __global__ void RRB_SEG_BOUNDS k_seg_write(const double* __restrict__ pts, const
                             const double* __restrict__ mtx, double flat_sq, const uint32_t* __restrict__ edge_off,
                             uint32_t edge_cap, Edge* __restrict__ edges,
                             const uint32_t* __restrict__ slot_clip_hi, const uint32_t* __restrict__ slot_clip_lo,
-                            int big_min = CURVE_BIG) {
+                            int big_min = CURVE_BIG, const BatchCounters* __restrict__ ctr = nullptr) {
+    if (SPLIT) n_slots = ctr->n_pieces;
     __shared__ double m[6];
     if (threadIdx.x < 6) m[threadIdx.x] = mtx[threadIdx.x];
     __syncthreads();
@@ -687,10 +692,33 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* sh, ui
     return wp + x - v;
 }
 
+// What becomes of a scan's total: stored at `total` (optional), and an error of
+// the batch when it passes `cap`, or when the 64-bit sum `wide` (optional) says
+// that it may have wrapped.
+struct ScanTotal {
+    uint32_t* total;
+    uint32_t cap, err_bit;
+    const unsigned long long* wide;
+    BatchCounters* ctr;
+    __device__ __forceinline__ void set(uint32_t t) const {
+        if (!total) return;
+        *total = t;
+        if (t > cap || (wide && *wide > 0x7FFFFFFFull)) atomicOr(&ctr->err, err_bit);
+    }
+};
+
+// n_ptr: the element count on the device (then n and per_block are not read).
+__device__ __forceinline__ void scan_range(uint32_t& n, uint32_t& per_block, const uint32_t* n_ptr) {
+    if (!n_ptr) return;
+    n = *n_ptr;
+    per_block = (n + gridDim.x - 1) / gridDim.x;
+}
+
 __global__ void k_scan_reduce(const uint32_t* __restrict__ in, uint32_t n, uint32_t per_block,
-                              uint32_t* __restrict__ block_sums) {
+                              uint32_t* __restrict__ block_sums, const uint32_t* __restrict__ n_ptr = nullptr) {
     __shared__ uint32_t sh[32];
-    uint32_t b0 = blockIdx.x * per_block;
+    scan_range(n, per_block, n_ptr);
+    uint32_t b0 = min(n, blockIdx.x * per_block);
     uint32_t b1 = min(n, b0 + per_block);
     uint32_t acc = 0;
     for (uint32_t i = b0 + threadIdx.x; i < b1; i += blockDim.x) acc += in[i];
@@ -704,19 +732,24 @@ __global__ void k_scan_reduce(const uint32_t* __restrict__ in, uint32_t n, uint3
     }
 }
 
-__global__ void k_scan_blocks(uint32_t* __restrict__ block_sums, uint32_t nb) {
+__global__ void k_scan_blocks(uint32_t* __restrict__ block_sums, uint32_t nb, ScanTotal out = ScanTotal{}) {
     __shared__ uint32_t sh[32];
     uint32_t v = threadIdx.x < nb ? block_sums[threadIdx.x] : 0u;
     uint32_t total;
     uint32_t ex = block_excl_scan(v, sh, total);
     if (threadIdx.x < nb) block_sums[threadIdx.x] = ex;
-    if (threadIdx.x == 0) block_sums[SCAN_MAX_BLOCKS] = total;
+    if (threadIdx.x == 0) {
+        block_sums[SCAN_MAX_BLOCKS] = total;
+        out.set(total);
+    }
 }
 
 __global__ void k_scan_down(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, uint32_t n,
-                            uint32_t per_block, const uint32_t* __restrict__ block_sums) {
+                            uint32_t per_block, const uint32_t* __restrict__ block_sums,
+                            const uint32_t* __restrict__ n_ptr = nullptr) {
     __shared__ uint32_t sh[32];
-    uint32_t b0 = blockIdx.x * per_block;
+    scan_range(n, per_block, n_ptr);
+    uint32_t b0 = min(n, blockIdx.x * per_block);
     uint32_t b1 = min(n, b0 + per_block);
     uint32_t carry = block_sums[blockIdx.x];
     for (uint32_t t0 = b0; t0 < b1; t0 += blockDim.x) {
@@ -728,6 +761,61 @@ __global__ void k_scan_down(const uint32_t* __restrict__ in, uint32_t* __restric
         carry += total;
     }
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = block_sums[SCAN_MAX_BLOCKS];
+}
+
+// Scans of up to SCAN_SMALL elements in one launch, an array per block (eight
+// elements a thread and step): three launches of a few microseconds each become
+// one, and two arrays that are ready together share it.
+constexpr uint32_t SCAN_SMALL = 16384;
+struct ScanJob {
+    const uint32_t* in;
+    uint32_t* out;
+    uint32_t n;
+    const uint32_t* n_ptr;
+    ScanTotal total;
+};
+struct ScanJobs {
+    ScanJob j[2];
+};
+
+__global__ void __launch_bounds__(1024) k_scan_jobs(const ScanJobs jobs) {
+    __shared__ uint32_t sh[32];
+    const ScanJob J = blockIdx.x ? jobs.j[1] : jobs.j[0];
+    const uint32_t n = J.n_ptr ? *J.n_ptr : J.n;
+    uint32_t carry = 0;
+    for (uint32_t t0 = 0; t0 < n; t0 += 8 * 1024) {
+        const uint32_t i0 = t0 + 8 * threadIdx.x;
+        uint32_t v[8], sum = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+            v[k] = i0 + k < n ? J.in[i0 + k] : 0u;
+            sum += v[k];
+        }
+        uint32_t total;
+        uint32_t at = carry + block_excl_scan(sum, sh, total);  // its barriers order the reads before the writes
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+            if (i0 + k < n) J.out[i0 + k] = at;
+            at += v[k];
+        }
+        carry += total;
+    }
+    if (threadIdx.x == 0) {
+        J.out[n] = carry;
+        J.total.set(carry);
+    }
+}
+
+// The row bounds of the edge groups, empty: 0x7f7f7f7f / 0x80808080 lie beyond
+// any AA row. With the sizes on the device this cannot be a memset.
+__global__ void k_init_groups(int32_t* __restrict__ gmin, int32_t* __restrict__ gmax,
+                              const BatchCounters* __restrict__ ctr) {
+    if (ctr->err) return;
+    const uint32_t n = ctr->n_edges / 32 + 1;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        gmin[i] = 0x7f7f7f7f;
+        gmax[i] = static_cast<int32_t>(0x80808080u);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -748,6 +836,7 @@ __global__ void RRB_BBOX_BOUNDS k_path_bbox(const uint32_t* __restrict__ piece_o
                             int chunk_rows, BatchCounters* __restrict__ ctr, int32_t* __restrict__ gmin,
                             int32_t* __restrict__ gmax, const int4* __restrict__ path_clip,
                             const int2* __restrict__ path_visit) {
+    if (ctr->err) return;  // a size beyond its buffer: nothing below is valid
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t warp_g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -960,7 +1049,13 @@ __device__ __forceinline__ uint32_t find_page_work(const PageGeom* pg, uint32_t 
 template <bool WRITE>
 __global__ void k_super_bin(const PathInfo* __restrict__ info, const PageGeom* __restrict__ pages, uint32_t n_pages,
                             uint32_t n_work, int stw, int sth, uint32_t* __restrict__ work_count,
-                            const uint32_t* __restrict__ work_off, uint32_t* __restrict__ super_list) {
+                            const uint32_t* __restrict__ work_off, uint32_t* __restrict__ super_list,
+                            uint32_t* __restrict__ chunk_live, const BatchCounters* __restrict__ ctr) {
+    if (ctr->err) return;  // a size beyond its buffer: nothing below is valid
+    if (WRITE) {  // k_tile_start marks the chunks it needs (four marks a word)
+        const uint32_t n = (ctr->n_chunks + 3) / 4;
+        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) chunk_live[i] = 0;
+    }
     int lane = threadIdx.x & 31;
     uint32_t warp_g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -1037,7 +1132,7 @@ __global__ void __launch_bounds__(START_WARPS * 32) k_tile_start(
     int rowmap, bool rgb, const uint32_t* __restrict__ chunk_off, uint32_t* __restrict__ tile_start,
     uint8_t* __restrict__ chunk_live, const BatchCounters* __restrict__ ctr) {
     __shared__ uint32_t ring_all[START_WARPS][START_RING];
-    if (ctr->solid == 0) return;
+    if (ctr->solid == 0 || ctr->err) return;
     const uint32_t lane = threadIdx.x & 31;
     uint32_t* ring = ring_all[threadIdx.x >> 5];
     const uint32_t nwarps = gridDim.x * START_WARPS;
@@ -1458,6 +1553,7 @@ __global__ void k_chunk_paths(const uint32_t* __restrict__ chunk_off, uint32_t n
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t warp_g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const bool all = ctr->solid == 0;
+    if (ctr->err) return;
     if (all && blockIdx.x == 0 && threadIdx.x == 0) ctr->live_chunks = chunk_off[n_paths];
     for (uint32_t p = warp_g; p < n_paths; p += nwarps) {
         const uint32_t c0 = chunk_off[p], c1 = chunk_off[p + 1];
@@ -1498,6 +1594,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_rows(
     uint32_t cell_cap, uint2* __restrict__ ovf, uint32_t ovf_cap, BatchCounters* __restrict__ ctr,
     const uint2* __restrict__ live, const int4* __restrict__ path_clip) {
     extern __shared__ __align__(16) int32_t rows_smem[];
+    if (ctr->err) return;
     constexpr int LIST = WARPS * KCAP * 32;
     auto sx0 = reinterpret_cast<int32_t (*)[KCAP * 32]>(rows_smem);
     auto sx1 = reinterpret_cast<int32_t (*)[KCAP * 32]>(rows_smem + LIST);
@@ -1744,6 +1841,7 @@ __global__ void k_recti(PathInfo* __restrict__ info, uint32_t n_paths, const Edg
                         const uint32_t* __restrict__ run_off, int4* __restrict__ runs, uint32_t* __restrict__ cells,
                         uint32_t cell_cap, BatchCounters* __restrict__ ctr, const int4* __restrict__ path_clip) {
     uint32_t nonterm = 0;
+    if (ctr->err || (WRITE && ctr->n_runs == 0)) return;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n_paths; p += gridDim.x * blockDim.x) {
         PathInfo P = info[p];
         if (P.paint & PI_SOLID) continue;  // hairline layers: runs from k_hl_count / k_hl_write
@@ -1952,6 +2050,7 @@ __global__ void __launch_bounds__(MID_WARPS * 32) k_groups_mid(
     __shared__ int32_t scn[MID_WARPS][MID_K * 4];
     __shared__ Edge sedge[MID_WARPS][32];
     __shared__ int32_t sns[MID_WARPS][4];
+    if (ctr->err) return;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t n_ovf = min(ctr->ovf_count, ovf_cap);
     uint32_t nonterm = 0;
@@ -2073,6 +2172,7 @@ __global__ void k_groups_slow(const PathInfo* __restrict__ info, const uint32_t*
     // (merging into the list's last entry as fill_intersections does). The
     // warp sorts the lists, lanes 0-3 walk them, lane 0 writes the cells.
     __shared__ int3 stage[SLOW_WARPS][4][32];
+    if (ctr->err & ~ERR_SCRATCH_CAP) return;  // every row asks for its scratch, so the next attempt knows the sum
     const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const uint32_t n_ovf = min(ctr->ovf2_count, ovf_cap);
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);

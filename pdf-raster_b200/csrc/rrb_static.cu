@@ -64,10 +64,10 @@ struct StaticHeader {
     BatchCounters ctr;
     double mtx[6];
     uint64_t off[2];
-    uint32_t page, pw, ph, pad0;
-    uint8_t rule, gray, alpha, pad1[5];
+    uint32_t page, pw, ph;
+    uint8_t rule, gray, alpha, pad;
     uint32_t path_pieces[2];
-    uint32_t rows[2], chunks[2];
+    uint32_t rows[1], chunks[1];
     uint32_t block[SCAN_MAX_BLOCKS + 1];
 };
 
