@@ -235,6 +235,17 @@ int upload(rrb_ctx* c, Scratch& s, const T* src, size_t count) {
     return RRB_OK;
 }
 
+// Small copies to and from page-locked memory go through a kernel: a copy
+// engine serves its queue in order, and behind the point uploads and page
+// downloads of a streamed batch a size of four bytes waits for megabytes: 9
+// pages from host memory in four ranges 15.6 -> 14.3 ms, one glyph 198 -> 180 us.
+int copy_words(rrb_ctx* c, const void* src, void* dst, size_t bytes) {
+    const uint32_t n = static_cast<uint32_t>(bytes / 4);
+    k_copy_words<<<grid_for(c, n, 128), 128, 0, c->stream>>>(static_cast<const uint32_t*>(src), static_cast<uint32_t*>(dst), n);
+    RRB_CUDA(c, cudaGetLastError());
+    return RRB_OK;
+}
+
 // A batch's counters as they stand at this point of the stream, into slot k of
 // the page-locked readback area; wait_counters waits for them.
 constexpr size_t kCounterSlot = 128;  // 32-bit words from one slot to the next, the first at word 128
@@ -242,8 +253,8 @@ static_assert(sizeof(BatchCounters) <= kCounterSlot * 4, "a slot holds the count
 
 int send_counters(rrb_ctx* c, int k) {
     if (!c->size_ev[k]) RRB_CUDA(c, cudaEventCreateWithFlags(&c->size_ev[k], cudaEventDisableTiming));
-    RRB_CUDA(c, cudaMemcpyAsync(c->h_read + (k + 1) * kCounterSlot, c->s_ctr.p, sizeof(BatchCounters),
-                                cudaMemcpyDeviceToHost, c->stream));
+    const int rc = copy_words(c, c->s_ctr.p, c->h_read + (k + 1) * kCounterSlot, sizeof(BatchCounters));
+    if (rc) return rc;
     RRB_CUDA(c, cudaEventRecord(c->size_ev[k], c->stream));
     return RRB_OK;
 }
@@ -257,7 +268,8 @@ int wait_counters(rrb_ctx* c, int k, BatchCounters& out) {
 
 int read_back(rrb_ctx* c, const void* dev, size_t bytes) {
     ++c->host_syncs;
-    RRB_CUDA(c, cudaMemcpyAsync(c->h_read, dev, bytes, cudaMemcpyDeviceToHost, c->stream));
+    const int rc = copy_words(c, dev, c->h_read, bytes);
+    if (rc) return rc;
     RRB_CUDA(c, cudaStreamSynchronize(c->stream));
     return RRB_OK;
 }
@@ -703,10 +715,12 @@ int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int
     const double flat_sq = B->flat_sq;
     const int4* pclip = B->has_clip ? as<int4>(B->clip) : nullptr;
     int rc;
-    if (cached && c->h_geom && c->geom_slot + n_pages <= c->h_geom_cap) {
+    if (c->h_geom && c->geom_slot + n_pages <= c->h_geom_cap) {
+        // Renders without cached sizes end with a wait, and waves with them have a
+        // slot each: the staging is free again when it is written.
         PageGeom* st = c->h_geom + c->geom_slot;
         std::memcpy(st, B->geom_h.data(), n_pages * sizeof(PageGeom));
-        RRB_CUDA(c, cudaMemcpyAsync(B->geom.p, st, n_pages * sizeof(PageGeom), cudaMemcpyHostToDevice, c->stream));
+        if ((rc = copy_words(c, st, B->geom.p, n_pages * sizeof(PageGeom)))) return rc;
     } else {
         RRB_CUDA(c, cudaMemcpyAsync(B->geom.p, B->geom_h.data(), n_pages * sizeof(PageGeom), cudaMemcpyHostToDevice,
                                     c->stream));
@@ -1300,6 +1314,22 @@ int run_pages(rrb_ctx* c, rrb_batch* B, uint32_t pg0, uint32_t pg1, uint8_t* are
 
 int run_resident_waves(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int rowmap);
 
+// Page-locked staging for the geometry of n_pages pages.
+void stage_geometry(rrb_ctx* c, uint32_t n_pages) {
+    if (c->h_geom_cap < n_pages) {
+        if (c->h_geom) cudaFreeHost(c->h_geom);
+        c->h_geom = nullptr;
+        c->h_geom_cap = 0;
+        void* h = nullptr;
+        if (cudaMallocHost(&h, std::max<size_t>(n_pages, 64) * sizeof(PageGeom)) == cudaSuccess) {
+            c->h_geom = static_cast<PageGeom*>(h);
+            c->h_geom_cap = static_cast<uint32_t>(std::max<size_t>(n_pages, 64));
+        } else {
+            cudaGetLastError();  // geometry then comes from pageable memory
+        }
+    }
+}
+
 int run_resident(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int rowmap) {
     if (B->trial_epoch != c->tuning_epoch) {
         // Plan the first phase of the trials: the tile shapes (the context's,
@@ -1415,18 +1445,7 @@ int run_resident_waves(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_le
             cudaGetLastError();  // no slots: every wave reads its sizes back
         }
     }
-    if (c->h_geom_cap < B->n_pages) {
-        if (c->h_geom) cudaFreeHost(c->h_geom);
-        c->h_geom = nullptr;
-        c->h_geom_cap = 0;
-        void* h = nullptr;
-        if (cudaMallocHost(&h, std::max<size_t>(B->n_pages, 64) * sizeof(PageGeom)) == cudaSuccess) {
-            c->h_geom = static_cast<PageGeom*>(h);
-            c->h_geom_cap = static_cast<uint32_t>(std::max<size_t>(B->n_pages, 64));
-        } else {
-            cudaGetLastError();  // geometry then comes from pageable memory
-        }
-    }
+    stage_geometry(c, B->n_pages);
     std::vector<uint32_t> done_plan{plan.front()}, deferred;
     for (size_t i = 0; i < n_waves; ++i) {
         const uint32_t slot = static_cast<uint32_t>(i);
@@ -1624,6 +1643,8 @@ struct HostPages {
 // ranges render.
 int run_streamed(rrb_ctx* c, const rrb_path_batch_params* h, rrb_batch* B, uint8_t* arena, size_t arena_len,
                  const HostPages* io = nullptr) {
+    stage_geometry(c, B->n_pages);
+    c->geom_slot = 0;
     if (!c->copy_stream) RRB_CUDA(c, cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
     if (io && !c->down_stream) RRB_CUDA(c, cudaStreamCreateWithFlags(&c->down_stream, cudaStreamNonBlocking));
     // Ranges of consecutive paths: a first one of about a tenth of the

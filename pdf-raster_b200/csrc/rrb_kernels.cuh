@@ -806,6 +806,11 @@ __global__ void __launch_bounds__(1024) k_scan_jobs(const ScanJobs jobs) {
     }
 }
 
+// n words between device memory and page-locked host memory, by the SMs.
+__global__ void k_copy_words(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, uint32_t n) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = src[i];
+}
+
 // The row bounds of the edge groups, empty: 0x7f7f7f7f / 0x80808080 lie beyond
 // any AA row. With the sizes on the device this cannot be a memset.
 __global__ void k_init_groups(int32_t* __restrict__ gmin, int32_t* __restrict__ gmax,
