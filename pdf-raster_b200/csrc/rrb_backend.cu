@@ -288,10 +288,8 @@ void preload_trial_kernels() {
 #define RRB_PRELOAD(...) cudaFuncGetAttributes(&a, reinterpret_cast<const void*>(__VA_ARGS__))
 #define RRB_PRELOAD_COMP(TW, TH)                      \
     do {                                              \
-        RRB_PRELOAD(k_composite<TW, TH, false, false>); \
-        RRB_PRELOAD(k_composite<TW, TH, false, true>);  \
-        RRB_PRELOAD(k_composite<TW, TH, true, false>);  \
-        RRB_PRELOAD(k_composite<TW, TH, true, true>);   \
+        RRB_PRELOAD(k_composite<TW, TH, false>);      \
+        RRB_PRELOAD(k_composite<TW, TH, true>);       \
     } while (0)
     RRB_PRELOAD_COMP(16, 16);
     RRB_PRELOAD_COMP(32, 32);
@@ -321,29 +319,21 @@ int launch_composite(rrb_ctx* c, int tw, int th, int grid, const PathInfo* info,
                      uint32_t n_pages, uint32_t n_tiles, const uint32_t* super_off, const uint32_t* super_list,
                      const uint32_t* row_off, const uint2* row_idx, const uint32_t* spans, const int4* runs,
                      uint8_t* arena, int rowmap, BatchCounters* ctr, const uint32_t* path_rgb,
-                     bool rectilinear, const uint32_t* tile_start) {
-#define RRB_COMP(TW, TH, RGB, FEW)                                                                           \
-    k_composite<TW, TH, RGB, FEW><<<grid, comp_threads(TW, TH), 0, c->stream>>>(                              \
+                     const uint32_t* tile_start) {
+#define RRB_COMP(TW, TH, RGB)                                                                                \
+    k_composite<TW, TH, RGB><<<grid, comp_threads(TW, TH), 0, c->stream>>>(                                   \
         info, geom, n_pages, n_tiles, SUPER, SUPER, super_off, super_list, row_off, row_idx, spans, runs, arena, \
         rowmap, ctr, path_rgb, tile_start)
-#define RRB_COMP_SHAPE(RGB, FEW)                                  \
-    do {                                                          \
-        if (tw == 64 && th == 16) RRB_COMP(64, 16, RGB, FEW);     \
-        else if (tw == 128 && th == 16) RRB_COMP(128, 16, RGB, FEW); \
-        else if (tw == 128 && th == 32) RRB_COMP(128, 32, RGB, FEW); \
-        else if (tw == 32 && th == 32) RRB_COMP(32, 32, RGB, FEW); \
-        else RRB_COMP(16, 16, RGB, FEW);                          \
+#define RRB_COMP_SHAPE(RGB)                                  \
+    do {                                                     \
+        if (tw == 64 && th == 16) RRB_COMP(64, 16, RGB);     \
+        else if (tw == 128 && th == 16) RRB_COMP(128, 16, RGB); \
+        else if (tw == 128 && th == 32) RRB_COMP(128, 32, RGB); \
+        else if (tw == 32 && th == 32) RRB_COMP(32, 32, RGB); \
+        else RRB_COMP(16, 16, RGB);                          \
     } while (0)
-    // Batches with rectilinear paths (rectangles) use the variant with the
-    // direct cell lookup for their rows; others keep the plain kernel, whose
-    // register allocation the extra path would disturb.
-    if (path_rgb) {
-        if (rectilinear) RRB_COMP_SHAPE(true, true);
-        else RRB_COMP_SHAPE(true, false);
-    } else {
-        if (rectilinear) RRB_COMP_SHAPE(false, true);
-        else RRB_COMP_SHAPE(false, false);
-    }
+    if (path_rgb) RRB_COMP_SHAPE(true);
+    else RRB_COMP_SHAPE(false);
 #undef RRB_COMP_SHAPE
 #undef RRB_COMP
     c->launches += 1;
@@ -1084,7 +1074,7 @@ int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int
                                as<uint32_t>(c->s_super_cnt), as<uint32_t>(c->s_super_list), as<uint32_t>(c->s_rows),
                                as<uint2>(c->s_row_idx), as<uint32_t>(c->s_spans), as<int4>(c->s_runs), arena,
                                rowmap, as<BatchCounters>(c->s_ctr), B->bpp == 3 ? as<uint32_t>(B->rgb) : nullptr,
-                               n_runs > 0, as<uint32_t>(c->s_tile_start))))
+                               as<uint32_t>(c->s_tile_start))))
         return rc;
     stage_end(c, 11);
     c->stats.paths = n_paths;
