@@ -72,16 +72,51 @@ __host__ __device__ __forceinline__ int32_t sat_i32_of_integral(double x) {
     if (x <= -2147483648.0) return INT32_MIN;
     return static_cast<int32_t>(x);
 }
-__host__ __device__ __forceinline__ int32_t splash_floor(double x) { return sat_i32_of_integral(floor(x)); }
+// On the device one conversion: to int32 it rounds down and saturates by itself
+// (infinities too), and takes a NaN double to INT32_MIN as this does.
+__host__ __device__ __forceinline__ int32_t splash_floor(double x) {
+#ifdef __CUDA_ARCH__
+    return __double2int_rd(x);
+#else
+    return sat_i32_of_integral(floor(x));
+#endif
+}
 
 // fp_from_f64 (crates/raster/src/scanner/mod.rs:51-66): truncating 16.16.
 __host__ __device__ __forceinline__ int32_t fp_from_f64(double x) {
     double fp = dmul(x, 65536.0);
+#ifdef __CUDA_ARCH__
+    return isnan(fp) ? 0 : __double2int_rz(fp);  // truncates and saturates
+#else
     if (fp >= 2147483647.0) return INT32_MAX;
     if (fp <= -2147483648.0) return INT32_MIN;
     if (isnan(fp)) return 0;
     return trunc_i32(fp);
+#endif
 }
+
+// round(fp) (halves away from zero) as int32, saturating, NaN to 0.
+__host__ __device__ __forceinline__ int32_t round_i32(double fp) {
+#ifdef __CUDA_ARCH__
+    // Below saturation the truncation and the rest are exact; beyond it the
+    // rest has fp's sign and is at least a half or not, and the sum must not wrap.
+    const int32_t t = __double2int_rz(fp);
+    const double rest = dsub(fp, static_cast<double>(t));
+    if (rest >= 0.5) return t == INT32_MAX ? t : t + 1;
+    if (rest <= -0.5) return t == INT32_MIN ? t : t - 1;
+    return isnan(fp) ? 0 : t;
+#else
+    if (fp >= 2147483647.0) return INT32_MAX;
+    if (fp <= -2147483648.0) return INT32_MIN;
+    if (isnan(fp)) return 0;
+    return static_cast<int32_t>(round(fp));
+#endif
+}
+
+// fmin / fmax where a is not NaN (a NaN b gives a; zeros of either sign are
+// equal for every use here).
+__host__ __device__ __forceinline__ double lesser(double a, double b) { return b < a ? b : a; }
+__host__ __device__ __forceinline__ double greater(double a, double b) { return b > a ? b : a; }
 
 __host__ __device__ __forceinline__ int32_t sat_i64_to_i32(long long v) {
     return v > INT32_MAX ? INT32_MAX : (v < INT32_MIN ? INT32_MIN : static_cast<int32_t>(v));
@@ -137,8 +172,8 @@ __host__ __device__ __forceinline__ Edge make_edge(double x0, double y0, double 
             e.row0 = 1;
             e.row1 = 0;
         }
-        e.a = splash_floor(fmin(sx0, sx1));
-        e.b = splash_floor(fmax(sx0, sx1));
+        e.a = splash_floor(lesser(sx0, sx1));
+        e.b = splash_floor(greater(sx0, sx1));
         return e;
     }
     bool vert = bx0 == bx1;
@@ -149,14 +184,7 @@ __host__ __device__ __forceinline__ Edge make_edge(double x0, double y0, double 
         t = y0; y0 = y1; y1 = t;
         flipped = true;
     }
-    int32_t dxdy_fp;
-    {
-        double fp = dmul(dxdy, 65536.0);
-        if (fp >= 2147483647.0) dxdy_fp = INT32_MAX;
-        else if (fp <= -2147483648.0) dxdy_fp = INT32_MIN;
-        else if (isnan(fp)) dxdy_fp = 0;
-        else dxdy_fp = static_cast<int32_t>(round(fp));
-    }
+    const int32_t dxdy_fp = round_i32(dmul(dxdy, 65536.0));
     x0 = dmul(x0, 4.0);
     y0 = dmul(y0, 4.0);
     x1 = dmul(x1, 4.0);
@@ -169,7 +197,7 @@ __host__ __device__ __forceinline__ Edge make_edge(double x0, double y0, double 
         e.a = 0;
         return e;
     }
-    double sy_min = fmin(y0, y1), sy_max = fmax(y0, y1);
+    double sy_min = lesser(y0, y1), sy_max = greater(y0, y1);
     int32_t r0 = max(splash_floor(sy_min), clip_lo);
     int32_t r1 = min(splash_floor(sy_max), clip_hi);
     e.row0 = r0;
@@ -181,7 +209,7 @@ __host__ __device__ __forceinline__ Edge make_edge(double x0, double y0, double 
         return e;
     }
     double x_base = dfma(y0, -dxdy, x0);
-    double sxmin = fmin(x0, x1), sxmax = fmax(x0, x1);
+    double sxmin = lesser(x0, x1), sxmax = greater(x0, x1);
     e.cmin = fp_from_f64(sxmin);
     e.cmax = fp_from_f64(sxmax);
     double r0d = static_cast<double>(r0);
