@@ -341,6 +341,21 @@ int launch_composite(rrb_ctx* c, int tw, int th, int grid, const PathInfo* info,
     return RRB_OK;
 }
 
+// Binning geometry ((supertile x path block) work items) of pages whose path
+// ranges are set; returns the number of work items.
+uint64_t set_binning(std::vector<PageGeom>& geom, uint32_t block = BIN_BLOCK) {
+    uint64_t work = 0;
+    for (PageGeom& G : geom) {
+        const uint64_t paths = G.path_end - G.path_begin;
+        G.nsx = (G.w + SUPER - 1) / SUPER;
+        G.bin_block = block;
+        G.nblk = static_cast<uint32_t>(std::max<uint64_t>(1, (paths + block - 1) / block));
+        G.work_base = static_cast<uint32_t>(work);
+        work += static_cast<uint64_t>(G.nsx) * ((G.h + SUPER - 1) / SUPER) * G.nblk;
+    }
+    return work > BIN_MAX_ITEMS && block == BIN_BLOCK ? set_binning(geom, BIN_BLOCK_LARGE) : work;
+}
+
 // Host-side checks of a batch (the params.validate() of the reference,
 // crates/gpu/src/backend/params.rs:57,334), plus the page geometry the
 // kernels need. No device access.
@@ -381,7 +396,6 @@ int validate_batch(const rrb_path_batch_params* h, size_t arena_len, uint32_t tw
         G.ntx = (w + tw - 1) / tw;
         G.nsx = (w + SUPER - 1) / SUPER;
         G.tile_base = static_cast<uint32_t>(tiles);
-        G.super_base = static_cast<uint32_t>(supers);
         tiles += static_cast<uint64_t>(G.ntx) * ((ht + th - 1) / th);
         supers += static_cast<uint64_t>(G.nsx) * ((ht + SUPER - 1) / SUPER);
     }
@@ -393,16 +407,14 @@ int validate_batch(const rrb_path_batch_params* h, size_t arena_len, uint32_t tw
         if (h->fill_rule[p] > max_rule) return msg = "fill_rule must be 0 or 1", RRB_ERR_INVARIANT;
         prev = pg;
     }
-    uint64_t p = 0, work = 0;
+    uint64_t p = 0;
     for (uint32_t pg = 0; pg < n_pages; ++pg) {
         PageGeom& G = geom[pg];
         G.path_begin = static_cast<uint32_t>(p);
         while (p < n_paths && h->path_page[p] == pg) ++p;
         G.path_end = static_cast<uint32_t>(p);
-        G.nblk = std::max<uint32_t>(1, (G.path_end - G.path_begin + BIN_BLOCK - 1) / BIN_BLOCK);
-        G.work_base = static_cast<uint32_t>(work);
-        work += static_cast<uint64_t>(G.nsx) * ((G.h + SUPER - 1) / SUPER) * G.nblk;
     }
+    const uint64_t work = set_binning(geom);
     if (tiles >= (1ull << 31) || supers >= (1ull << 31) || work >= (1ull << 31))
         return msg = "too many tiles", RRB_ERR_INVARIANT;
     supers = work;  // binning work items
@@ -1166,21 +1178,6 @@ int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int
     return RRB_OK;
 }
 
-// Binning geometry (supertiles, (supertile x path block) work items) of pages
-// whose path ranges are already set.
-void set_binning(std::vector<PageGeom>& geom, uint64_t& supers_out) {
-    uint64_t supers = 0, work = 0;
-    for (PageGeom& G : geom) {
-        G.nsx = (G.w + SUPER - 1) / SUPER;
-        G.super_base = static_cast<uint32_t>(supers);
-        supers += static_cast<uint64_t>(G.nsx) * ((G.h + SUPER - 1) / SUPER);
-        G.nblk = std::max<uint32_t>(1, (G.path_end - G.path_begin + BIN_BLOCK - 1) / BIN_BLOCK);
-        G.work_base = static_cast<uint32_t>(work);
-        work += static_cast<uint64_t>(G.nsx) * ((G.h + SUPER - 1) / SUPER) * G.nblk;
-    }
-    supers_out = work;
-}
-
 void release_scratch(rrb_ctx* c) {
     cudaStreamSynchronize(c->stream);
     Scratch* all[] = {&c->s_pieces, &c->s_clip, &c->s_edge_off, &c->s_edges, &c->s_info, &c->s_rows, &c->s_chunks,
@@ -1243,7 +1240,7 @@ int make_wave(rrb_ctx* c, rrb_batch* B, uint32_t pg0, uint32_t pg1, rrb_batch* W
         G.path_begin -= pb;
         G.path_end -= pb;
     }
-    set_binning(W->geom_h, W->supers);
+    W->supers = set_binning(W->geom_h);
     W->page_pt.clear();
     return RRB_OK;
 }
@@ -1557,7 +1554,7 @@ int make_path_wave(rrb_ctx* c, rrb_batch* B, uint32_t pa, uint32_t pb, uint64_t 
         G.path_end = std::max(std::min(G.path_end, pb), pa) - pa;
         if (G.path_end < G.path_begin) G.path_end = G.path_begin;
     }
-    set_binning(W->geom_h, W->supers);
+    W->supers = set_binning(W->geom_h);
     W->page_pt.clear();
     W->plan.clear();
     return RRB_OK;

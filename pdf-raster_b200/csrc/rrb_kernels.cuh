@@ -1112,21 +1112,24 @@ struct PageGeom {
     uint32_t w, h;
     uint32_t path_begin, path_end;
     uint32_t tile_base, ntx;       // tiles of this page start at tile_base, ntx per row
-    uint32_t super_base, nsx;      // supertiles start at super_base, nsx per row
-    uint32_t work_base, nblk;      // binning work items: (supertile, block of BIN_BLOCK paths)
+    uint32_t bin_block, nsx;       // paths per binning work item, supertiles per row
+    uint32_t work_base, nblk;      // binning work items: (supertile, block of bin_block paths)
     uint64_t offset;               // page byte offset in the arena
 };
 
 // Paths per binning work item: a warp takes 32 at a time, one load latency
 // each. 2,048 left a page's 17 blocks busy for 34 us with 2,000 paths; 256: 11.
-constexpr uint32_t BIN_BLOCK = 256;
+// Batches that would have more than 16 Mi items that way (64 MB of counts; the
+// device is full with a few thousand) keep 2,048, so that as large a batch as
+// ever can be counted.
+constexpr uint32_t BIN_BLOCK = 256, BIN_BLOCK_LARGE = 2048;
+constexpr uint64_t BIN_MAX_ITEMS = 1ull << 24;
 
-__device__ __forceinline__ uint32_t find_page_by(const PageGeom* pg, uint32_t n_pages, uint32_t idx, bool super) {
-    uint32_t lo = 0, hi = n_pages;  // last page with base <= idx
+__device__ __forceinline__ uint32_t find_page_tile(const PageGeom* pg, uint32_t n_pages, uint32_t t) {
+    uint32_t lo = 0, hi = n_pages;  // last page with base <= t
     while (hi - lo > 1) {
         uint32_t mid = (lo + hi) >> 1;
-        uint32_t b = super ? pg[mid].super_base : pg[mid].tile_base;
-        if (b <= idx) lo = mid;
+        if (pg[mid].tile_base <= t) lo = mid;
         else hi = mid;
     }
     return lo;
@@ -1166,8 +1169,8 @@ __global__ void k_super_bin(const PathInfo* __restrict__ info, const PageGeom* _
         uint32_t sl = local / G.nblk, blk = local % G.nblk;
         int32_t sx = static_cast<int32_t>(sl % G.nsx), sy = static_cast<int32_t>(sl / G.nsx);
         int32_t x0 = sx * stw, x1 = x0 + stw - 1, y0 = sy * sth, y1 = y0 + sth - 1;
-        uint32_t pb = G.path_begin + blk * BIN_BLOCK;
-        uint32_t pe = min(G.path_end, pb + BIN_BLOCK);
+        uint32_t pb = G.path_begin + blk * G.bin_block;
+        uint32_t pe = min(G.path_end, pb + G.bin_block);
         uint32_t cnt = 0;
         uint32_t base = WRITE ? work_off[q] : 0u;
         for (uint32_t j = pb; j < pe; j += 32) {
@@ -1237,7 +1240,7 @@ __global__ void __launch_bounds__(START_WARPS * 32) k_tile_start(
     uint32_t* ring = ring_all[threadIdx.x >> 5];
     const uint32_t nwarps = gridDim.x * START_WARPS;
     for (uint32_t t = blockIdx.x * START_WARPS + (threadIdx.x >> 5); t < n_tiles; t += nwarps) {
-        const PageGeom G = pages[find_page_by(pages, n_pages, t, false)];
+        const PageGeom G = pages[find_page_tile(pages, n_pages, t)];
         const uint32_t lt = t - G.tile_base;
         const int32_t X0 = static_cast<int32_t>(lt % G.ntx) * tw, Y0 = static_cast<int32_t>(lt / G.ntx) * th;
         const int32_t TX1 = min(X0 + tw, static_cast<int32_t>(G.w)) - 1;
@@ -2747,7 +2750,7 @@ __global__ void __launch_bounds__(comp_threads(TW, TH), comp_ctas_per_sm(TW, TH)
         return next_tile;
     };
     for (uint32_t t = take(); t < n_tiles; t = take()) {
-        const uint32_t pg = find_page_by(pages, n_pages, t, false);
+        const uint32_t pg = find_page_tile(pages, n_pages, t);
         const PageGeom G = pages[pg];
         const uint32_t lt = t - G.tile_base;
         const int tx = static_cast<int>(lt % G.ntx), ty = static_cast<int>(lt / G.ntx);
