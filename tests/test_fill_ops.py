@@ -172,6 +172,35 @@ def test_aa_fill_matches_aa_fill_cpu(backend, oracle, fill_cases, rule):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("w,clusters", [
+    (1024, [(0, 33, 20)]), (1024, [(0, 33, 70)]), (1024, [(900, 1024, 40)]), (1024, [(130, 250, 120), (600, 602, 18)]),
+    (1024, [(0, 1024, 400)]), (1024, [(127, 129, 17), (383.5, 384.5, 90), (1020, 1030, 30)]),
+    (1030, [(1000, 1030, 64)]), (300, [(0, 300, 300)]), (40, [(3, 9, 65), (30, 40, 17)]), (9, [(0, 9, 200)]),
+    (1, [(0, 1, 40)]), (2048, [(500, 520, 33), (1024, 1040, 16), (1500, 1501, 17)])])
+def test_aa_fill_dense_parts(backend, oracle, w, clusters):
+    """Sample lines with more crossings than a list keeps in some columns and few or none in the others."""
+    rng = np.random.default_rng(w + len(clusters))
+    h, segs = 5, []
+    for x0, x1, n in clusters + [(0, w, 6)]:
+        x, up = rng.uniform(x0, x1, n), rng.integers(0, 2, n).astype(bool)
+        y0, y1 = np.full(n, -1.0), np.where(rng.random(n) < 0.8, h + 1.0, rng.uniform(0, h, n))
+        segs.append(np.stack([x, np.where(up, y0, y1), x + rng.uniform(-2, 2, n), np.where(up, y1, y0)], 1))
+    segs = np.concatenate(segs).astype(np.float32)
+    for rule in (0, 1):
+        exp = oracle.aa_fill_cpu(segs, 0.0, 0.0, w, h, eo=bool(rule))
+        sb, cb = _dev(backend, segs), backend.alloc_device(w * h)
+        try:
+            backend.upload_async(cb, np.full(w * h, 77, np.uint8))
+            _run(backend, lambda: backend.record_aa_fill(sb, len(segs), cb, w, h, rule))
+            got = np.empty(w * h, np.uint8)
+            backend.wait_download(backend.download_async(cb, got))
+            assert np.array_equal(got, exp.ravel())
+        finally:
+            backend.free_device(sb)
+            backend.free_device(cb)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("w,h,n", [(1, 1, 3), (3, 5, 9), (63, 4, 40), (1023, 3, 60), (1024, 5, 60), (1025, 4, 200),
                                    (2051, 3, 400), (130, 5, 1100), (1100, 2, 1400)])
 def test_aa_fill_chunk_edges(backend, oracle, w, h, n):
