@@ -124,9 +124,9 @@ GLYPH_DRAM_BYTES_PER_SEGMENT = {
 # DRAM bytes per page pixel of the composite on the mixed batch:
 # dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of
 # k_composite<128, 16> on page 0 of the batch alone (3508x4961, 17,589 paths;
-# its cells and row index larger than L2), scaled to a launch by its pixels.
+# the page's last layers stay in L2), scaled to a launch by its pixels.
 MIXED_DRAM_BYTES_PER_PIXEL = {
-    "composite": (92_113_664 + 15_584_256) / (3508 * 4961),
+    "composite": (16_695_808 + 1_127_680) / (3508 * 4961),
 }
 
 
@@ -470,7 +470,8 @@ def run_rrb(args, rank, local, world):
     alg = {
         # page read + written once, each coverage cell (4 B) and pixel-row index entry (8 B) read once
         "composite": 2 * px + 4 * stats["spans"] + 8 * stats["row_groups"],
-        # each edge record (32 B) read once, pixel-row index (8 B/entry) and cells (4 B) written once
+        # each edge record (32 B) read once, pixel-row index (8 B/entry) and cells (4 B) written once (an
+        # upper bound where later layers hide rows: those are not built)
         "rows": 32 * stats["segments"] + 8 * stats["row_groups"] + 4 * stats["spans"],
         # path points (16 B) + flags read, edge records written
         "seg_write": 17 * scene.n_pts + 32 * stats["segments"],

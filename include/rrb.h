@@ -460,7 +460,8 @@ typedef struct {
     uint64_t host_ns;                       /* host time of the call before its first kernel: validation,
                                                stroke outlines, staging and enqueued uploads */
     uint64_t row_groups;                    /* pixel-row index entries written by the row stage */
-    uint64_t host_syncs;                    /* times the call waited on its stream for a device-side size */
+    uint64_t host_syncs;                    /* times the call waited for device-side sizes (between its stages, or
+                                               behind them where a small batch is launched whole) */
     uint64_t tile_w, tile_h;                /* tile shape of the render */
     uint64_t row_shape;                     /* row-stage shape (entries per AA row x warps x edge groups per
                                                warp): 0 = 12x8x2, 1 = 16x4x2, 2 = 12x8x1, 3 = 8x16x2,
