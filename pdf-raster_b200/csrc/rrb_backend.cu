@@ -822,7 +822,7 @@ int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int
     k_seg_write_big<<<c->sm_count * 16, 128, 0, c->stream>>>(
         as<double>(B->pts), as<uint2>(c->s_pieces), as<double>(B->mtx), flat_sq, as<uint32_t>(c->s_big),
         as<BatchCounters>(c->s_ctr), as<uint32_t>(c->s_edge_off), static_cast<uint32_t>(n_edges),
-        as<Edge>(c->s_edges), as<uint32_t>(c->s_clip), clip_lo, as<uint8_t>(c->s_lanes), lane_cap);
+        as<Edge>(c->s_edges), as<uint32_t>(c->s_clip), clip_lo, as<uint8_t>(c->s_lanes), lane_cap, big_min);
     c->launches += 2;
     stage_end(c, 3);
     const int chunk_rows = 32;
