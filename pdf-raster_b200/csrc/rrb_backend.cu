@@ -53,6 +53,8 @@ constexpr int kRowShapes = 5;
 constexpr uint64_t kLaneCountCurves = 1ull << 22;  // big curves whose lane counts are kept (128 MiB)
 constexpr uint32_t kLongWalk = 64;    // path points from which a warp walks a path
 constexpr uint64_t kFewPaths = 4096;  // paths up to which warps walk them all (one launch)
+constexpr uint64_t kMaxGroups = 0x3FFFFFFF;  // pixel rows (groups of four AA rows) of a wave's paths
+constexpr uint64_t kMaxRuns = 0x7FFFFFFF;    // row runs of its rectilinear paths and hairlines
 constexpr int SUPER = 256;      // supertile edge in pixels (a multiple of every tile shape)
 
 }  // namespace
@@ -207,7 +209,7 @@ int scan_u32(rrb_ctx* c, const ScanJob& job, uint64_t bound) {
     uint32_t nb = std::min<uint32_t>(SCAN_MAX_BLOCKS, std::max<uint32_t>(1, (n + 4095) / 4096));
     uint32_t per = (n + nb - 1) / nb;
     nb = (n + per - 1) / per;
-    k_scan_reduce<<<nb, SCAN_THREADS, 0, c->stream>>>(job.in, job.n, per, bs, job.n_ptr);
+    k_scan_reduce<<<nb, SCAN_THREADS, 0, c->stream>>>(job.in, job.n, per, bs, job.n_ptr, job.total);
     k_scan_blocks<<<1, 1024, 0, c->stream>>>(bs, nb, job.total);
     k_scan_down<<<nb, SCAN_THREADS, 0, c->stream>>>(job.in, job.out, job.n, per, bs, job.n_ptr);
     c->launches += 3;
@@ -751,9 +753,9 @@ int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int
         long_walk);
     c->launches += 1;
     RRB_CUDA(c, cudaGetLastError());
-    constexpr uint32_t kNoCap = 0xFFFFFFFFu;
     uint32_t* path_pieces = as<uint32_t>(c->s_path_pieces);
-    if ((rc = scan_u32(c, ScanJob{path_pieces, path_pieces, NP, nullptr, ScanTotal{&ctr->n_pieces, kNoCap, 0, nullptr, ctr}},
+    if ((rc = scan_u32(c, ScanJob{path_pieces, path_pieces, NP, nullptr,
+                                  ScanTotal{&ctr->n_pieces, MAX_OFFSET, ERR_EDGE_CAP, ctr}},
                        NP)))
         return rc;
     if (sized && (rc = read_back(c, path_pieces + NP, sizeof(uint32_t)))) return rc;
@@ -791,18 +793,28 @@ int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int
     RRB_CUDA(c, cudaGetLastError());
     stage(c, 2);
     // What a count may reach (free: what its buffers hold; the kernels behind
-    // stop at the error otherwise).
-    auto cap32 = [](uint64_t v) { return static_cast<uint32_t>(std::min<uint64_t>(v, 0xFFFFFF00ull)); };
+    // stop at the error otherwise; sized: what 32-bit offsets hold, and the
+    // render ends where the count is read).
+    auto cap32 = [](uint64_t v) { return static_cast<uint32_t>(std::min<uint64_t>(v, MAX_OFFSET)); };
+    BatchCounters hs;
+    auto read_sizes = [&]() -> int {
+        if (int r = read_back(c, ctr, sizeof(BatchCounters))) return r;
+        std::memcpy(&hs, c->h_read, sizeof hs);
+        if (hs.err)
+            return set_err(c, RRB_ERR_POOL_EXHAUSTED,
+                           "batch needs more than 2^32 segments, pixel rows, supertile entries or row runs");
+        return RRB_OK;
+    };
     const uint64_t free_edges = std::min<uint64_t>(c->s_edges.cap / sizeof(Edge), (c->s_groups.cap / 8 - 2) * 32);
     uint32_t* edge_off = as<uint32_t>(c->s_edge_off);
     if ((rc = scan_u32(c, ScanJob{edge_off, edge_off, 0, &ctr->n_pieces,
-                                  ScanTotal{&ctr->n_edges, free ? cap32(free_edges) : kNoCap, ERR_EDGE_CAP, nullptr, ctr}},
+                                  ScanTotal{&ctr->n_edges, cap32(free ? free_edges : MAX_OFFSET), ERR_EDGE_CAP, ctr}},
                        n_pieces)))
         return rc;
     stage_end(c, 2);
     if (free && (rc = send_counters(c, 0))) return rc;
-    if (sized && (rc = read_back(c, &ctr->n_edges, sizeof(uint32_t)))) return rc;
-    const uint64_t n_edges = cached ? ws->n_edges : free ? cap32(free_edges) : c->h_read[0];
+    if (sized && (rc = read_sizes())) return rc;
+    const uint64_t n_edges = cached ? ws->n_edges : free ? cap32(free_edges) : hs.n_edges;
     // ---- stage 2: edges, path boxes, row/chunk offsets, supertile bins
     if ((rc = ensure(c, c->s_edges, std::max<uint64_t>(1, n_edges) * sizeof(Edge)))) return rc;
     if ((rc = ensure(c, c->s_info, n_paths * sizeof(PathInfo)))) return rc;
@@ -848,18 +860,16 @@ int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int
     stage_end(c, 4);
     RRB_CUDA(c, cudaGetLastError());
     stage(c, 5);
-    // 32-bit offsets: refused where the paths' AA rows could have wrapped them
-    // (free: rendered again with sizes, which checks as it always has).
     const uint64_t free_groups = std::min(std::min(c->s_row_idx.cap, c->s_ovf.cap), c->s_ovf2.cap) / sizeof(uint2);
     const uint64_t free_chunks = std::min<uint64_t>(c->s_chunk_path.cap / sizeof(uint2), c->s_chunk_live.cap - 4);
-    const unsigned long long* rows_wide = free ? &ctr->aa_rows : nullptr;
     uint32_t *path_rows = as<uint32_t>(c->s_rows), *path_chunks = as<uint32_t>(c->s_chunks);
     if ((rc = scan_u32_pair(
              c,
              ScanJob{path_rows, path_rows, NP, nullptr,
-                     ScanTotal{&ctr->n_groups, free ? cap32(free_groups) : kNoCap, ERR_ROW_CAP, rows_wide, ctr}},
+                     ScanTotal{&ctr->n_groups, cap32(free ? std::min<uint64_t>(free_groups, kMaxGroups) : MAX_OFFSET),
+                               ERR_ROW_CAP, ctr}},
              ScanJob{path_chunks, path_chunks, NP, nullptr,
-                     ScanTotal{&ctr->n_chunks, free ? cap32(free_chunks) : kNoCap, ERR_ROW_CAP, rows_wide, ctr}})))
+                     ScanTotal{&ctr->n_chunks, cap32(free ? free_chunks : MAX_OFFSET), ERR_ROW_CAP, ctr}})))
         return rc;
     stage_end(c, 5);
     const uint32_t NSUP = static_cast<uint32_t>(supers);
@@ -881,10 +891,10 @@ int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int
     if ((rc = scan_u32_pair(
              c,
              ScanJob{super_cnt, super_cnt, NSUP, nullptr,
-                     ScanTotal{&ctr->n_pairs, free ? cap32(c->s_super_list.cap / 4) : kNoCap, ERR_SUPER_CAP, nullptr, ctr}},
+                     ScanTotal{&ctr->n_pairs, cap32(free ? c->s_super_list.cap / 4 : MAX_OFFSET), ERR_SUPER_CAP, ctr}},
              ScanJob{path_runs, path_runs, NP, nullptr,
-                     ScanTotal{&ctr->n_runs, free ? cap32(c->s_runs.cap / sizeof(int4)) : kNoCap, ERR_RUN_CAP,
-                               free ? &ctr->hl_rows : nullptr, ctr}})))
+                     ScanTotal{&ctr->n_runs, cap32(free ? std::min<uint64_t>(c->s_runs.cap / sizeof(int4), kMaxRuns) : MAX_OFFSET),
+                               ERR_RUN_CAP, ctr}})))
         return rc;
     stage_end(c, 7);
     if (free && (rc = send_counters(c, 1))) return rc;
@@ -903,9 +913,7 @@ int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int
         n_runs = c->s_runs.cap / sizeof(int4);
         raw_entries = hl_rows = 0;
     } else {
-        if ((rc = read_back(c, ctr, sizeof(BatchCounters)))) return rc;
-        BatchCounters hs;
-        std::memcpy(&hs, c->h_read, sizeof hs);
+        if ((rc = read_sizes())) return rc;
         n_groups = hs.n_groups;
         n_chunks = hs.n_chunks;
         n_pairs = hs.n_pairs;
@@ -913,8 +921,7 @@ int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int
         raw_entries = hs.raw_entries;
         hl_rows = hs.hl_rows;
     }
-    // The run offsets were scanned in 32 bits: refuse totals that could wrap.
-    if (!free && (hl_rows > 0x7FFFFFFFull || n_runs > 0x7FFFFFFFull))
+    if (!free && (hl_rows > kMaxRuns || n_runs > kMaxRuns))
         return set_err(c, RRB_ERR_POOL_EXHAUSTED, "batch needs more than 2^31 row runs");
     // ---- stage 3: rows -> coverage cells. An AA row with m merged entries
     // yields at most m/2 + 1 spans, and a pixel row at most 2 cells per span
@@ -923,7 +930,7 @@ int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int
     uint64_t cell_cap = 2 * raw_entries + 4 * aa_rows + hl_rows + 1024;
     if (free) cell_cap = std::min<uint64_t>(c->s_spans.cap / sizeof(uint32_t), 0xFFFFFF00ull);
     if (cell_cap > 0xFFFFFF00ull) return set_err(c, RRB_ERR_POOL_EXHAUSTED, "batch needs more than 2^32 cells");
-    if (!free && n_groups > 0x3FFFFFFFull) return set_err(c, RRB_ERR_POOL_EXHAUSTED, "batch needs more than 2^30 pixel rows");
+    if (!free && n_groups > kMaxGroups) return set_err(c, RRB_ERR_POOL_EXHAUSTED, "batch needs more than 2^30 pixel rows");
     if (!free) {
         if ((rc = ensure(c, c->s_row_idx, std::max<uint64_t>(1, n_groups) * sizeof(uint2)))) return rc;
         if ((rc = ensure(c, c->s_spans, cell_cap * sizeof(uint32_t)))) return rc;

@@ -796,20 +796,43 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* sh, ui
     return wp + x - v;
 }
 
+// The largest total that 32-bit offsets may reach: the loops over a list step
+// past its end by up to a grid of warps, which must not wrap either.
+constexpr uint32_t MAX_OFFSET = 0xFFFF0000u;
+
+// Whether offsets whose 64-bit total this is are what they say, and within cap
+// entries (at most MAX_OFFSET).
+__host__ __device__ __forceinline__ bool scan_fits(unsigned long long total, uint32_t cap) { return total <= cap; }
+
 // What becomes of a scan's total: stored at `total` (optional), and an error of
-// the batch when it passes `cap`, or when the 64-bit sum `wide` (optional) says
-// that it may have wrapped.
+// the batch when it passes `cap`. The scans add in 32 bits and keep the sum in
+// 64 beside that: one page may hold 2^30 points, whose segments, rows and
+// supertile entries go beyond 2^32, and offsets that wrapped would be taken for
+// a batch that fits.
 struct ScanTotal {
     uint32_t* total;
     uint32_t cap, err_bit;
-    const unsigned long long* wide;
     BatchCounters* ctr;
-    __device__ __forceinline__ void set(uint32_t t) const {
+    __device__ __forceinline__ void fail() const {
+        if (total) atomicOr(&ctr->err, err_bit);
+    }
+    __device__ __forceinline__ void set(unsigned long long t) const {
         if (!total) return;
-        *total = t;
-        if (t > cap || (wide && *wide > 0x7FFFFFFFull)) atomicOr(&ctr->err, err_bit);
+        *total = static_cast<uint32_t>(t);
+        if (!scan_fits(t, cap)) fail();
     }
 };
+
+// The sum of v over the block, on thread 0 (sh: a word per warp).
+__device__ __forceinline__ unsigned long long block_sum(unsigned long long v, unsigned long long* sh) {
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = 0;
+    if (threadIdx.x == 0)
+        for (uint32_t w = 0; w < blockDim.x >> 5; ++w) v += sh[w];
+    return v;
+}
 
 // n_ptr: the element count on the device (then n and per_block are not read).
 __device__ __forceinline__ void scan_range(uint32_t& n, uint32_t& per_block, const uint32_t* n_ptr) {
@@ -819,32 +842,32 @@ __device__ __forceinline__ void scan_range(uint32_t& n, uint32_t& per_block, con
 }
 
 __global__ void k_scan_reduce(const uint32_t* __restrict__ in, uint32_t n, uint32_t per_block,
-                              uint32_t* __restrict__ block_sums, const uint32_t* __restrict__ n_ptr = nullptr) {
-    __shared__ uint32_t sh[32];
+                              uint32_t* __restrict__ block_sums, const uint32_t* __restrict__ n_ptr = nullptr,
+                              ScanTotal out = ScanTotal{}) {
+    __shared__ unsigned long long sh[32];
     scan_range(n, per_block, n_ptr);
     uint32_t b0 = min(n, blockIdx.x * per_block);
     uint32_t b1 = min(n, b0 + per_block);
-    uint32_t acc = 0;
+    unsigned long long acc = 0;
     for (uint32_t i = b0 + threadIdx.x; i < b1; i += blockDim.x) acc += in[i];
-    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
-    __syncthreads();
+    acc = block_sum(acc, sh);
     if (threadIdx.x == 0) {
-        uint32_t t = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sh[w];
-        block_sums[blockIdx.x] = t;
+        block_sums[blockIdx.x] = static_cast<uint32_t>(acc);
+        if (acc >> 32) out.fail();  // wrapped in this block already: k_scan_blocks sees what is left
     }
 }
 
 __global__ void k_scan_blocks(uint32_t* __restrict__ block_sums, uint32_t nb, ScanTotal out = ScanTotal{}) {
     __shared__ uint32_t sh[32];
+    __shared__ unsigned long long sh_sum[32];
     uint32_t v = threadIdx.x < nb ? block_sums[threadIdx.x] : 0u;
     uint32_t total;
     uint32_t ex = block_excl_scan(v, sh, total);
     if (threadIdx.x < nb) block_sums[threadIdx.x] = ex;
+    const unsigned long long sum = block_sum(v, sh_sum);
     if (threadIdx.x == 0) {
         block_sums[SCAN_MAX_BLOCKS] = total;
-        out.set(total);
+        out.set(sum);
     }
 }
 
@@ -884,9 +907,11 @@ struct ScanJobs {
 
 __global__ void __launch_bounds__(1024) k_scan_jobs(const ScanJobs jobs) {
     __shared__ uint32_t sh[32];
+    __shared__ unsigned long long sh_sum[32];
     const ScanJob J = blockIdx.x ? jobs.j[1] : jobs.j[0];
     const uint32_t n = J.n_ptr ? *J.n_ptr : J.n;
     uint32_t carry = 0;
+    unsigned long long mine = 0;
     for (uint32_t t0 = 0; t0 < n; t0 += 8 * 1024) {
         const uint32_t i0 = t0 + 8 * threadIdx.x;
         uint32_t v[8], sum = 0;
@@ -894,6 +919,7 @@ __global__ void __launch_bounds__(1024) k_scan_jobs(const ScanJobs jobs) {
         for (uint32_t k = 0; k < 8; ++k) {
             v[k] = i0 + k < n ? J.in[i0 + k] : 0u;
             sum += v[k];
+            mine += v[k];
         }
         uint32_t total;
         uint32_t at = carry + block_excl_scan(sum, sh, total);  // its barriers order the reads before the writes
@@ -904,9 +930,10 @@ __global__ void __launch_bounds__(1024) k_scan_jobs(const ScanJobs jobs) {
         }
         carry += total;
     }
+    mine = block_sum(mine, sh_sum);
     if (threadIdx.x == 0) {
         J.out[n] = carry;
-        J.total.set(carry);
+        J.total.set(mine);
     }
 }
 
