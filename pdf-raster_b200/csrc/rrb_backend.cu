@@ -805,7 +805,9 @@ int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int
                            "batch needs more than 2^32 segments, pixel rows, supertile entries or row runs");
         return RRB_OK;
     };
-    const uint64_t free_edges = std::min<uint64_t>(c->s_edges.cap / sizeof(Edge), (c->s_groups.cap / 8 - 2) * 32);
+    // (Bounds of n edges take (n + 31) / 32 + 1 groups: what a render by size
+    // was given always holds the same batch launched whole.)
+    const uint64_t free_edges = std::min<uint64_t>(c->s_edges.cap / sizeof(Edge), (c->s_groups.cap / 8 - 1) * 32);
     uint32_t* edge_off = as<uint32_t>(c->s_edge_off);
     if ((rc = scan_u32(c, ScanJob{edge_off, edge_off, 0, &ctr->n_pieces,
                                   ScanTotal{&ctr->n_edges, cap32(free ? free_edges : MAX_OFFSET), ERR_EDGE_CAP, ctr}},
