@@ -681,12 +681,17 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
     int rc = run_pipeline(c, B, arena, arena_len, rowmap, ws, slot, free, &retry);
     // Its buffers per point are bounds: without room for them, by size too.
     if (free && rc == RRB_ERR_OUT_OF_MEMORY) {
+        ++c->host_syncs;
         RRB_CUDA(c, cudaStreamSynchronize(c->stream));
         retry = true;
     }
     if (!retry) return rc;
     c->wait_pages_up = pages_pending;
-    return run_pipeline(c, B, arena, arena_len, rowmap, ws, slot, false, nullptr);
+    const uint64_t launches = c->launches, host_syncs = c->host_syncs;
+    rc = run_pipeline(c, B, arena, arena_len, rowmap, ws, slot, false, nullptr);
+    c->stats.kernel_launches += launches;  // what the call launched and waited for in both
+    c->stats.host_syncs += host_syncs;
+    return rc;
 }
 
 int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int rowmap, WaveSizes* ws, uint32_t slot,
@@ -1121,6 +1126,7 @@ int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int
         for (int k = 0; k < 3; ++k) {
             if ((rc = wait_counters(c, k, hc))) return rc;
             if (hc.err) {
+                if (k < 2) ++c->host_syncs;
                 RRB_CUDA(c, cudaEventSynchronize(c->size_ev[2]));  // before any buffer grows
                 *retry = true;
                 return RRB_OK;
