@@ -171,9 +171,8 @@ __global__ void k_hl_count(const double* __restrict__ pts, const uint64_t* __res
                            int rowmap, PathInfo* __restrict__ info, uint32_t* __restrict__ run_count,
                            BatchCounters* __restrict__ ctr) {
     __shared__ double m[6];
-    if (ctr->err) return;
     if (threadIdx.x < 6) m[threadIdx.x] = mtx[threadIdx.x];
-    __syncthreads();
+    if (block_stops(ctr)) return;
     unsigned long long total = 0;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n_paths; p += gridDim.x * blockDim.x) {
         if (rule[p] != RULE_HAIRLINE) continue;
@@ -229,9 +228,8 @@ __global__ void k_hl_write(const double* __restrict__ pts, const uint64_t* __res
                            PathInfo* __restrict__ info, int4* __restrict__ runs, uint32_t* __restrict__ cells,
                            uint32_t cell_cap, BatchCounters* __restrict__ ctr) {
     __shared__ double m[6];
-    if (ctr->err) return;
     if (threadIdx.x < 6) m[threadIdx.x] = mtx[threadIdx.x];
-    __syncthreads();
+    if (block_stops(ctr)) return;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
     for (uint32_t p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); p < n_paths; p += warps) {

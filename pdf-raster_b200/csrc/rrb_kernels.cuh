@@ -97,6 +97,17 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
     return m;
 }
 
+// Whether an error of the batch stops a kernel here, decided by a whole warp or
+// block at once (the latter a barrier): a kernel that can set the error itself
+// may find it set by another block between two threads' reads, and threads
+// that leave alone would be missed at the next shuffle or barrier.
+__device__ __forceinline__ bool warp_stops(const BatchCounters* ctr, uint32_t bits = ~0u) {
+    return __any_sync(0xffffffffu, (ctr->err & bits) != 0);
+}
+__device__ __forceinline__ bool block_stops(const BatchCounters* ctr) {
+    return __syncthreads_or(threadIdx.x == 0 && ctr->err != 0);
+}
+
 // f(p), by whole blocks, for the paths that is_long picks: a block looks at up
 // to 32 paths at a time (a lane of its first warp each), so that finding none
 // costs a page of 150,000 paths a few loads per block, and at fewer where there
@@ -1735,7 +1746,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_rows(
     uint32_t cell_cap, uint2* __restrict__ ovf, uint32_t ovf_cap, BatchCounters* __restrict__ ctr,
     const uint2* __restrict__ live, const int4* __restrict__ path_clip) {
     extern __shared__ __align__(16) int32_t rows_smem[];
-    if (ctr->err) return;
+    if (warp_stops(ctr)) return;
     constexpr int LIST = WARPS * KCAP * 32;
     auto sx0 = reinterpret_cast<int32_t (*)[KCAP * 32]>(rows_smem);
     auto sx1 = reinterpret_cast<int32_t (*)[KCAP * 32]>(rows_smem + LIST);
@@ -2191,7 +2202,7 @@ __global__ void __launch_bounds__(MID_WARPS * 32) k_groups_mid(
     __shared__ int32_t scn[MID_WARPS][MID_K * 4];
     __shared__ Edge sedge[MID_WARPS][32];
     __shared__ int32_t sns[MID_WARPS][4];
-    if (ctr->err) return;
+    if (warp_stops(ctr)) return;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t n_ovf = min(ctr->ovf_count, ovf_cap);
     uint32_t nonterm = 0;
@@ -2313,7 +2324,7 @@ __global__ void k_groups_slow(const PathInfo* __restrict__ info, const uint32_t*
     // (merging into the list's last entry as fill_intersections does). The
     // warp sorts the lists, lanes 0-3 walk them, lane 0 writes the cells.
     __shared__ int3 stage[SLOW_WARPS][4][32];
-    if (ctr->err & ~ERR_SCRATCH_CAP) return;  // every row asks for its scratch, so the next attempt knows the sum
+    if (warp_stops(ctr, ~ERR_SCRATCH_CAP)) return;  // every row asks for its scratch, so the next attempt knows the sum
     const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const uint32_t n_ovf = min(ctr->ovf2_count, ovf_cap);
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);

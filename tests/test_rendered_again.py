@@ -111,6 +111,7 @@ def _growing(rng):
     yield "pairs", P(rng, specks, w, h)
     yield "cells", P(rng, combs, w, h)
     yield "hairline runs", P(rng, lines, w, h)
+    yield "hairline cells", P(rng, combs + lines, w, h)  # the combs' cells first, then hairlines until none are left
 
 
 @pytest.mark.parametrize("form", ["gray", "clipped rgb"])
@@ -145,4 +146,4 @@ def test_a_batch_that_does_not_fit_is_rendered_again(rrb_lib, oracle, form):
                     again.add(name)
             assert st["host_syncs"] < by_size["host_syncs"]
             be.free_device(pages)
-    assert {"edges", "rows", "overflow rows", "runs", "pairs", "hairline runs"} <= again
+    assert {"edges", "rows", "overflow rows", "runs", "pairs", "hairline runs", "hairline cells"} <= again
