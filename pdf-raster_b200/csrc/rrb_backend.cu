@@ -116,6 +116,11 @@ struct rrb_ctx {
     // by its trials (0: none yet, 64x16), the default of batches uploaded per
     // call on this context until another batch settles or the tuning changes.
     uint32_t settled_tw = 0, settled_th = 0;
+    // Whole launches (run_resident_one): batches of this many points and more ran out
+    // of memory that way, and scratch sized by points instead of pieces is held.
+    uint64_t whole_limit = UINT64_MAX;
+    bool bounds_held = false;
+    bool rendering = false;                   // scratch is in use
     cudaEvent_t size_ev[3] = {nullptr, nullptr, nullptr};  // counters read back behind the launches (send_counters)
     cudaEvent_t trial_ev[2] = {nullptr, nullptr};  // timing of a resident batch's trial render
 };
@@ -137,11 +142,19 @@ int cuda_err(rrb_ctx* c, cudaError_t e, const char* what) {
         if (e__ != cudaSuccess) return cuda_err(ctx, e__, #call); \
     } while (0)
 
+bool give_back_bounds(rrb_ctx* c);
+
 int dev_alloc(rrb_ctx* c, size_t bytes, void** out) {
+    // Scratch that only holds bounds is no reason to refuse anything.
+    if (c->budget && c->used + bytes > c->budget) give_back_bounds(c);
     if (c->budget && c->used + bytes > c->budget)
         return set_err(c, RRB_ERR_OUT_OF_MEMORY,
                        "device allocation of " + std::to_string(bytes) + " bytes exceeds the budget");
     cudaError_t e = cudaMalloc(out, bytes);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        if (give_back_bounds(c)) e = cudaMalloc(out, bytes);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         return set_err(c, RRB_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e));
@@ -154,6 +167,20 @@ void dev_free(rrb_ctx* c, void* p, size_t bytes) {
     if (!p) return;
     cudaFree(p);
     c->used -= std::min<uint64_t>(c->used, bytes);
+}
+
+// Between renders: frees the scratch that whole launches sized by points (some
+// 65 bytes a point where a third of that by pieces would do). True if any was held.
+bool give_back_bounds(rrb_ctx* c) {
+    if (!c->bounds_held || c->rendering) return false;
+    cudaStreamSynchronize(c->stream);
+    for (Scratch* x : {&c->s_pieces, &c->s_clip, &c->s_clip_lo, &c->s_edge_off, &c->s_big, &c->s_lanes}) {
+        dev_free(c, x->p, x->cap);
+        x->p = nullptr;
+        x->cap = 0;
+    }
+    c->bounds_held = false;
+    return true;
 }
 
 // Grow a scratch buffer to at least `bytes` (x1.25 headroom); contents are not kept.
@@ -657,6 +684,8 @@ int batch_upload(rrb_ctx* c, const rrb_path_batch_params* h, rrb_batch* B, const
 // paths under clips 812 -> 692. Larger batches gain nothing by it.
 constexpr uint64_t kFreePoints = 2ull << 20;
 
+void release_scratch(rrb_ctx* c);
+
 // The pipeline over a device-resident batch into the device page arena.
 // ws: the wave's cached sizes (see WaveSizes), or nullptr. When they match,
 // every stage is launched without waiting on the stream, and the counters
@@ -673,23 +702,37 @@ int run_resident_one(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len,
     // Batches uploaded per call only: a kept batch pays for its waits once, and
     // launches exactly what its sizes ask for from then on. The buffers sized by
     // counts must exist (some render has sized them).
-    const bool free = B == c->tmp_batch && B->n_pts <= kFreePoints && c->s_edges.p && c->s_groups.p && c->s_row_idx.p && c->s_ovf.p &&
+    const bool free = B == c->tmp_batch && B->n_pts <= kFreePoints && B->n_pts < c->whole_limit && c->s_edges.p && c->s_groups.p && c->s_row_idx.p && c->s_ovf.p &&
                       c->s_ovf2.p && c->s_spans.p && c->s_super_list.p && c->s_runs.p && c->s_chunk_path.p &&
                       c->s_chunk_live.p;
     bool retry = false;
     const bool pages_pending = c->wait_pages_up;
+    c->rendering = true;
     int rc = run_pipeline(c, B, arena, arena_len, rowmap, ws, slot, free, &retry);
-    // Its buffers per point are bounds: without room for them, by size too.
+    uint64_t launches = 0, host_syncs = 0;  // of the attempts before the last
+    auto by_size = [&]() {
+        launches += c->launches;
+        host_syncs += c->host_syncs;
+        c->wait_pages_up = pages_pending;
+        return run_pipeline(c, B, arena, arena_len, rowmap, ws, slot, false, nullptr);
+    };
     if (free && rc == RRB_ERR_OUT_OF_MEMORY) {
+        // Its buffers per point are bounds: without room for them, by size too.
+        c->whole_limit = B->n_pts;
         ++c->host_syncs;
-        RRB_CUDA(c, cudaStreamSynchronize(c->stream));
-        retry = true;
+        if (cudaStreamSynchronize(c->stream) == cudaSuccess) retry = true;
     }
-    if (!retry) return rc;
-    c->wait_pages_up = pages_pending;
-    const uint64_t launches = c->launches, host_syncs = c->host_syncs;
-    rc = run_pipeline(c, B, arena, arena_len, rowmap, ws, slot, false, nullptr);
-    c->stats.kernel_launches += launches;  // what the call launched and waited for in both
+    if (retry) rc = by_size();
+    if (retry && rc == RRB_ERR_OUT_OF_MEMORY) {
+        // Nor for the sizes beside the bounds: by size from nothing, as if the
+        // batch had never been launched whole.
+        c->whole_limit = std::min(c->whole_limit, B->n_pts);
+        cudaGetLastError();
+        release_scratch(c);
+        rc = by_size();
+    }
+    c->rendering = false;
+    c->stats.kernel_launches += launches;  // what the call launched and waited for in all attempts
     c->stats.host_syncs += host_syncs;
     return rc;
 }
@@ -794,6 +837,7 @@ int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int
                                                             as<BatchCounters>(c->s_ctr), as<uint32_t>(c->s_edge_off),
                                                             as<uint8_t>(c->s_lanes), lane_cap);
     c->launches += 2;
+    if (free) c->bounds_held = true;
     stage_end(c, 1);
     RRB_CUDA(c, cudaGetLastError());
     stage(c, 2);
@@ -1195,6 +1239,7 @@ int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int
 
 void release_scratch(rrb_ctx* c) {
     cudaStreamSynchronize(c->stream);
+    c->bounds_held = false;
     Scratch* all[] = {&c->s_pieces, &c->s_clip, &c->s_edge_off, &c->s_edges, &c->s_info, &c->s_rows, &c->s_chunks,
                       &c->s_super_cnt, &c->s_super_list, &c->s_tile_start, &c->s_chunk_live, &c->s_big, &c->s_lanes, &c->s_row_idx, &c->s_spans, &c->s_ovf, &c->s_scratch,
                       &c->s_groups, &c->s_slots, &c->s_path_pieces, &c->s_ovf2, &c->s_run_off, &c->s_runs,
@@ -1270,12 +1315,16 @@ constexpr uint64_t kWavePoints = 40ull << 20;
 int run_pages(rrb_ctx* c, rrb_batch* B, uint32_t pg0, uint32_t pg1, uint8_t* arena, size_t arena_len, int rowmap,
               rrb_batch_stats& acc, int depth, std::vector<uint32_t>& done_plan, WaveSizes* ws = nullptr,
               uint32_t slot = 0) {
-    int rc;
-    if (pg0 == 0 && pg1 == B->n_pages) {
-        rc = run_resident_one(c, B, arena, arena_len, rowmap, ws, slot);
-    } else {
-        rc = make_wave(c, B, pg0, pg1, c->wave_batch);
-        if (!rc) rc = run_resident_one(c, c->wave_batch, arena, arena_len, rowmap, ws, slot);
+    auto render = [&]() {
+        if (pg0 == 0 && pg1 == B->n_pages) return run_resident_one(c, B, arena, arena_len, rowmap, ws, slot);
+        const int r = make_wave(c, B, pg0, pg1, c->wave_batch);
+        return r ? r : run_resident_one(c, c->wave_batch, arena, arena_len, rowmap, ws, slot);
+    };
+    int rc = render();
+    if (rc == RRB_ERR_OUT_OF_MEMORY && c->bounds_held) {  // beside scratch that holds bounds: once more from nothing
+        cudaGetLastError();
+        release_scratch(c);
+        rc = render();
     }
     if (rc == RRB_OK) {
         const rrb_batch_stats& s = c->stats;
@@ -1579,8 +1628,16 @@ int make_path_wave(rrb_ctx* c, rrb_batch* B, uint32_t pa, uint32_t pb, uint64_t 
 // is split in two (its composite had not run, so the pages are untouched).
 int run_path_range(rrb_ctx* c, rrb_batch* B, const uint64_t* path_pt_off, uint32_t pa, uint32_t pb, uint8_t* arena,
                    size_t arena_len, int rowmap, rrb_batch_stats& acc, int depth) {
-    int rc = make_path_wave(c, B, pa, pb, path_pt_off[pa], path_pt_off[pb], c->wave_batch);
-    if (!rc) rc = run_resident_one(c, c->wave_batch, arena, arena_len, rowmap);
+    auto render = [&]() {
+        const int r = make_path_wave(c, B, pa, pb, path_pt_off[pa], path_pt_off[pb], c->wave_batch);
+        return r ? r : run_resident_one(c, c->wave_batch, arena, arena_len, rowmap);
+    };
+    int rc = render();
+    if (rc == RRB_ERR_OUT_OF_MEMORY && c->bounds_held) {  // as in run_pages
+        cudaGetLastError();
+        release_scratch(c);
+        rc = render();
+    }
     if (rc == RRB_OK) {
         const rrb_batch_stats& s = c->stats;
         acc.paths += s.paths;
@@ -1961,6 +2018,7 @@ int rrb_free_device(rrb_ctx* c, rrb_buf* b) {
     const rrb_host::DeviceScope dev_scope(c->device);
     cudaStreamSynchronize(c->stream);
     dev_free(c, b->p, b->len);
+    c->whole_limit = UINT64_MAX;
     delete b;
     return RRB_OK;
 }
@@ -2189,6 +2247,7 @@ int rrb_batch_free(rrb_ctx* c, rrb_batch* B) {
     const rrb_host::DeviceScope dev_scope(c->device);
     cudaStreamSynchronize(c->stream);
     free_batch_bufs(c, B);
+    c->whole_limit = UINT64_MAX;
     delete B;
     return RRB_OK;
 }
