@@ -810,6 +810,7 @@ int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int
     // A path has at most one piece per point.
     const uint64_t n_pieces = cached ? ws->n_pieces : free ? n_pts : c->h_read[0];
     const uint32_t NPC = static_cast<uint32_t>(n_pieces);
+    if (free) c->bounds_held = true;  // also where one of them then finds no room
     if ((rc = ensure(c, c->s_pieces, std::max<uint64_t>(1, n_pieces) * sizeof(uint2)))) return rc;
     if ((rc = ensure(c, c->s_clip, std::max<uint64_t>(1, n_pieces) * sizeof(uint32_t)))) return rc;
     if (pclip && (rc = ensure(c, c->s_clip_lo, std::max<uint64_t>(1, n_pieces) * sizeof(uint32_t)))) return rc;
@@ -837,7 +838,6 @@ int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int
                                                             as<BatchCounters>(c->s_ctr), as<uint32_t>(c->s_edge_off),
                                                             as<uint8_t>(c->s_lanes), lane_cap);
     c->launches += 2;
-    if (free) c->bounds_held = true;
     stage_end(c, 1);
     RRB_CUDA(c, cudaGetLastError());
     stage(c, 2);
