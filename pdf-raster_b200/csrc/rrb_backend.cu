@@ -986,7 +986,6 @@ int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int
         if ((rc = ensure(c, c->s_row_idx, std::max<uint64_t>(1, n_groups) * sizeof(uint2)))) return rc;
         if ((rc = ensure(c, c->s_spans, cell_cap * sizeof(uint32_t)))) return rc;
         if ((rc = ensure(c, c->s_ovf, std::max<uint64_t>(1, n_groups) * sizeof(uint2)))) return rc;
-        if ((rc = ensure(c, c->s_ovf2, std::max<uint64_t>(1, n_groups) * sizeof(uint2)))) return rc;
         if ((rc = ensure(c, c->s_super_list, std::max<uint64_t>(1, n_pairs) * sizeof(uint32_t)))) return rc;
         if ((rc = ensure(c, c->s_runs, std::max<uint64_t>(1, n_runs) * sizeof(int4)))) return rc;
         if ((rc = ensure(c, c->s_chunk_live, n_chunks + 8))) return rc;
@@ -1000,6 +999,10 @@ int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int
         most_chunks = std::min(most_chunks, n_chunks);
     }
     if ((rc = ensure(c, c->s_tile_start, tiles * sizeof(uint32_t)))) return rc;
+    // The list of the rows that the overflow rows' own lists cannot hold: here only
+    // for batches launched whole later on, so left out where it finds no room.
+    const size_t ovf2_bytes = std::max<uint64_t>(1, n_groups) * sizeof(uint2);
+    if (sized && ensure(c, c->s_ovf2, ovf2_bytes)) c->err.clear();
     stage(c, 8);
     k_super_bin<true><<<grid_for(c, supers * 32, 256), 256, 0, c->stream>>>(
         as<PathInfo>(c->s_info), as<PageGeom>(B->geom), n_pages, NSUP, SUPER, SUPER, nullptr,
@@ -1071,6 +1074,7 @@ int run_pipeline(rrb_ctx* c, rrb_batch* B, uint8_t* arena, size_t arena_len, int
     uint64_t mid = cached ? ws->mid : free ? std::min<uint64_t>(8 * most_chunks, n_groups) : std::min<uint64_t>(hc.ovf_count, n_groups);
     uint64_t slow = 0, slow_need = 0;
     if (mid) {
+        if (!free && (rc = ensure(c, c->s_ovf2, ovf2_bytes))) return rc;
         stage(c, 10);
         k_groups_mid<<<grid_for(c, mid * 32, MID_WARPS * 32, 16), MID_WARPS * 32, 0, c->stream>>>(
             as<PathInfo>(c->s_info), as<uint32_t>(c->s_rows), as<Edge>(c->s_edges), gmin, gmax,

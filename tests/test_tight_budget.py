@@ -64,3 +64,17 @@ def test_bounds_are_given_back(rrb_lib, rest, want, fits):
         assert np.array_equal(_record(be, rrb_lib, s, pages), first)
         be.free_device(buf)
         assert np.array_equal(_record(be, rrb_lib, s, pages), first)
+
+
+def test_the_second_overflow_list_is_not_needed_without_overflow_rows(rrb_lib, oracle):
+    s = rrb_lib.Scene(kind=1, seed=19, n_paths=3000, page_w=1200, page_h=900)
+    exp = s.blank_arena()
+    oracle.render_scene(s, exp, threads=4)
+    with rrb_lib.B200Backend(0) as be:
+        _record(be, rrb_lib, s, be.alloc_device(s.arena_bytes))
+        need, st = be.detect_vram_budget().used_bytes, be.last_batch_stats()
+    assert st["row_overflows"] == 0
+    with rrb_lib.B200Backend(0, mem_budget=need - 8 * st["row_groups"]) as be:  # 10 bytes a row with the headroom
+        pages = be.alloc_device(s.arena_bytes)
+        for _ in range(2):
+            assert np.array_equal(_record(be, rrb_lib, s, pages), exp)
