@@ -23,8 +23,9 @@
 // A tile whose [start, start + count) runs past the records buffer is
 // treated as empty instead of being read out of bounds.
 //
-// record_tile_fill_segs takes the same segments as aa_fill: up to 32,768 of them
-// go straight to coverage (k_tile_fill_segs); more build the records on the
+// record_tile_fill_segs takes the same segments as aa_fill: where that is the
+// faster way (tile_scan_pays) they go straight to coverage (k_tile_fill_segs);
+// more of them, or larger windows, build the records on the
 // device (build_tile_records, fill.rs:82-264: count, write in segment order,
 // stable radix sort by tile key, per-tile ranges by binary search), then run
 // tile_fill. Neither builds or uploads records on the host.
@@ -874,10 +875,20 @@ int check_segs(rrb_ctx* c, const rrb_buf* segs, uint32_t n) {
     return RRB_OK;
 }
 
-// Segments up to which rrb_record_tile_fill_segs scans them per tile row. The
-// scan grows with segments x tile rows, the sort with segments alone: 64 us
-// against 189 at 14,752 segments, and at 33,772 the sort takes 180.
+// Whether every CTA scanning all segments beats sorting their records, from
+// the sizes alone. The scan costs 2.1 ps per segment and CTA and 0.5 ns per
+// tile, the sort some 100 us and 1 ns per tile. Whole calls of short segments
+// spread over the window, scan / sorted records in us: 1,024 x 1,024 and 14,752
+// segments 70 / 143, 32,768 98 / 200; 2,048 x 2,048, 32,768 170 / 230; 4,096 x
+// 4,096, 14,752 221 / 234, 32,768 411 / 395; 8,192 x 8,192, 2,048 198 / 414, 8,192
+// 417 / 421, 32,768 1,304 / 617; 16,384 x 16,384, 2,048 681 / 1,221, 8,192 1,465 /
+// 1,242. Windows of a few tiles leave a CTA or two with everything in either
+// form, and the fill's chain per record is the shorter one: 18,432 segments in 17
+// x 17 5,535 / 5,096, 5,760 in 40 x 30 357 / 453.
 constexpr uint32_t kTileScanSegs = 1u << 15;
+constexpr bool tile_scan_pays(uint32_t n, uint64_t row_ctas, uint64_t tiles) {
+    return n <= kTileScanSegs && n <= 4096 * tiles && n * row_ctas <= (48ull << 20) + 300 * tiles;
+}
 
 int launch_tile_fill(rrb_ctx* c, const TileRec* recs, uint64_t n_recs, const uint32_t* starts,
                      const uint32_t* counts, uint32_t w, uint32_t h, int eo, uint8_t* cov) {
@@ -1051,7 +1062,7 @@ int rrb_record_tile_fill_segs(rrb_ctx* c, const rrb_aa_fill_params* p, uint64_t*
     auto ctas = [&](uint32_t t) { return static_cast<uint64_t>(gh) * ((gw + t - 1) / t); };
     while (group_tiles > 1 && ctas(group_tiles) < static_cast<uint64_t>(sm)) group_tiles /= 2;
     const uint64_t row_ctas = ctas(group_tiles);
-    if (n <= kTileScanSegs && row_ctas <= 0x7FFFFFFFull && n * (2ull * gh + gw) < (1ull << 31)) {
+    if (tile_scan_pays(n, row_ctas, tiles) && row_ctas <= 0x7FFFFFFFull && n * (2ull * gh + gw) < (1ull << 31)) {
         if ((rc = rrb_ctx_fill_scratch(c, 0, 8, &v_off))) return rc;
         auto* count = static_cast<unsigned long long*>(v_off);
         if (n_records) FILL_CUDA(c, cudaMemsetAsync(count, 0, 8, s));
