@@ -38,7 +38,7 @@ def _short(n, w, h, seed):
 
 @pytest.mark.parametrize("w,h,n,by_records", [
     (17, 16, 8192, False), (17, 16, 8193, True), (300, 200, 32768, False), (300, 200, 32769, True),
-    (4096, 4096, 17087, False), (4096, 4096, 17088, True), (8192, 8192, 4096, False), (8192, 8192, 32768, True)])
+    (4096, 4096, 17088, False), (4096, 4096, 17089, True), (8192, 8192, 4096, False), (8192, 8192, 32768, True)])
 def test_the_sizes_choose_the_route(rrb_lib, oracle, w, h, n, by_records):
     segs = _short(n, w, h, n)
     recs, starts, counts, gw = oracle.build_tile_records(segs, 0.0, 0.0, w, h)
