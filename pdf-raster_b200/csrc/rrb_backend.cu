@@ -1884,6 +1884,13 @@ int rrb_ctx_fill_scratch(rrb_ctx* c, int k, size_t bytes, void** out) {
     return RRB_OK;
 }
 
+// Up to 512 bytes of device memory as they stand at this point of the stream (one wait).
+int rrb_ctx_read(rrb_ctx* c, const void* dev, size_t bytes, void* out) {
+    const int rc = read_back(c, dev, bytes);
+    if (!rc) std::memcpy(out, c->h_read, bytes);
+    return rc;
+}
+
 extern "C" {
 
 const char* rrb_version(void) { return "rrb 0.1 sm_100a"; }

@@ -48,6 +48,7 @@ bool rrb_ctx_page_open(const rrb_ctx* c);
 int rrb_ctx_fail(rrb_ctx* c, int code, const char* msg);
 int rrb_ctx_sm_count(const rrb_ctx* c);
 int rrb_ctx_fill_scratch(rrb_ctx* c, int k, size_t bytes, void** out);
+int rrb_ctx_read(rrb_ctx* c, const void* dev, size_t bytes, void* out);
 
 namespace {
 
@@ -645,6 +646,107 @@ __global__ void __launch_bounds__(TF_THREADS) k_tile_fill(const TileRec* __restr
 // areas in the busiest tile row.
 constexpr int TSF_NT = 256, TSF_TILES = 16, TSF_CAP = 1024;
 static_assert(TSF_NT == TF_THREADS && TSF_CAP == 4 * TSF_NT, "a pixel of a tile per thread, four segments at a time");
+struct TsfWork {
+    unsigned long long records;  // of all tile rows
+    uint32_t leave, pad;         // the sorted records are the faster way (k_tile_load): nothing is written
+};
+
+// Whether the contents are for the scan, by one CTA before it. Where some tile
+// rows have many records the chain of their CTAs is the scan's time (0.6 to 1 us
+// for each that all eight warps walk; 1.05 ns of the whole chip for each record
+// and tile), while the sorted records cost 0.7 ns each and a chain of 0.19 to
+// 0.35 us in their tile. So a sample of the segments is added up by tile row, each as
+// its pairs of pixel rows x tiles in a row, assumed even over the row's groups.
+// Scan / sorted records in us: 1,024 x 1,024, 32,768 long segments 3,293 /
+// 1,142, 8,192 860 / 434; all in 28 pixel rows of it, 32,768 884 / 220, 8,192 247 /
+// 134; 2,048 x 2,048, 32,768 long ones 2,957 / 2,033. With the look, whole calls:
+// 1,164, 457, 240, 156 and 2,061; 14,752 short ones 70 -> 65. It costs 5 us,
+// won back by reading its answer with the count; a call that leaves pays for the
+// wait too.
+constexpr uint32_t TL_THREADS = 512;  // and entries of the load, a tile row (or 2^shift of them) each
+constexpr uint32_t TL_PICKS = 2;       // segments looked at per thread
+__global__ void __launch_bounds__(TL_THREADS) k_tile_load(const float4* __restrict__ segs, uint32_t n_segs, uint32_t grid_w,
+                                                          uint32_t grid_h, uint32_t height, uint32_t groups,
+                                                          TsfWork* __restrict__ work) {
+    __shared__ uint32_t step[TL_THREADS + 1];  // load of an entry, less that of the one before
+    __shared__ uint32_t part[TL_THREADS / 32], peaks[TL_THREADS / 32];
+    __shared__ float2 recs_of[TL_THREADS / 32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    // Each pick is one out of `per` consecutive segments and stands for them all: those of
+    // an outline lie in the same rows, where all of them would add to the same
+    // words in turn (13 us of 14,000 segments).
+    const uint32_t per = (n_segs + TL_PICKS * TL_THREADS - 1) / (TL_PICKS * TL_THREADS), picks = n_segs / per;
+    float4 s[TL_PICKS];
+#pragma unroll
+    for (uint32_t j = 0; j < TL_PICKS; ++j) {
+        const uint32_t i = tid + j * TL_THREADS;
+        s[j] = i < picks ? segs[i * per + __umulhi(i * 2654435761u, per)] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    uint32_t shift = 0;
+    while (((grid_h - 1) >> shift) >= TL_THREADS) ++shift;
+    step[tid] = 0;
+    if (tid == 0) step[TL_THREADS] = 0;
+    __syncthreads();
+    float recs = 0.0f, walked = 0.0f;  // records; pairs of pixel rows that they touch
+    const float bottom = static_cast<float>(height), wide = static_cast<float>(min(grid_w, 255u));
+#pragma unroll
+    for (uint32_t j = 0; j < TL_PICKS; ++j) {
+        const float y0 = fmaxf(fminf(s[j].y, s[j].w), 0.0f), y1 = fminf(fmaxf(s[j].y, s[j].w), bottom);
+        if (!(y0 < y1)) continue;
+        const uint32_t r0 = min(static_cast<uint32_t>(y0) / TILE, grid_h - 1);
+        const uint32_t r1 = min(static_cast<uint32_t>(y1) / TILE, grid_h - 1);
+        const float tiles = fminf(fabsf(s[j].z - s[j].x) / fmaxf(fabsf(s[j].w - s[j].y), static_cast<float>(TILE)) + 1.0f, wide);
+        const uint32_t rows = r1 - r0 + 1;
+        // Pairs of pixel rows (a warp each) in a tile row: the mean of its rows.
+        const uint32_t pairs = (static_cast<uint32_t>(ceilf(0.5f * y1)) - static_cast<uint32_t>(0.5f * y0) + rows - 1) / rows;
+        recs += tiles * static_cast<float>(rows);
+        walked += tiles * static_cast<float>(rows * pairs);
+        uint32_t load = static_cast<uint32_t>(static_cast<float>(pairs) * tiles + 0.5f);
+        if (shift) load = max(1u, (load * min(rows, 1u << shift)) >> shift);  // the mean of the entry's rows
+        atomicAdd(&step[r0 >> shift], load);
+        atomicAdd(&step[(r1 >> shift) + 1], 0u - load);
+    }
+    __syncthreads();
+    uint32_t incl = step[tid];
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (static_cast<int>(lane) >= o) incl += t;
+    }
+    for (int o = 16; o; o >>= 1) {
+        recs += __shfl_xor_sync(0xffffffffu, recs, o);
+        walked += __shfl_xor_sync(0xffffffffu, walked, o);
+    }
+    if (lane == 31) part[w] = incl;
+    if (lane == 0) recs_of[w] = make_float2(recs, walked);
+    __syncthreads();
+    incl += __reduce_add_sync(0xffffffffu, lane < w ? part[lane] : 0u);
+    incl = __reduce_max_sync(0xffffffffu, incl);
+    if (lane == 0) peaks[w] = incl;
+    __syncthreads();
+    if (w) return;
+    const bool has = lane < TL_THREADS / 32;
+    const uint32_t peak = __reduce_max_sync(0xffffffffu, has ? peaks[lane] : 0u);
+    const float2 t = has ? recs_of[lane] : make_float2(0.0f, 0.0f);
+    float total = t.x;
+    walked = t.y;
+    for (int o = 16; o; o >>= 1) {
+        total += __shfl_xor_sync(0xffffffffu, total, o);
+        walked += __shfl_xor_sync(0xffffffffu, walked, o);
+    }
+    if (lane) return;
+    const float n = static_cast<float>(n_segs), of = n / static_cast<float>(picks);
+    const float tiles = static_cast<float>(grid_w) * static_cast<float>(grid_h);
+    const float row = of * static_cast<float>(peak) / 8.0f;  // records of the fullest row that a warp walks
+    // In its tile a sorted record is looked at by every warp: 0.19 us of the chain, 0.35 if all walk it.
+    const float in_tile = fmaxf(350.0f, 1520.0f * total / fmaxf(walked, 1.0f));
+    total *= of;
+    const float scan = 2.1e-3f * n * static_cast<float>(grid_h) * static_cast<float>(groups) + 0.5f * tiles +
+                       fmaxf(750.0f * row / static_cast<float>(groups), 1.05f * total);
+    const float sorted = 1e5f + 2.2f * n + tiles + 0.7f * total + in_tile * row / static_cast<float>(grid_w);
+    work->records = 0;
+    work->leave = scan > 1.15f * sorted + 2e4f ? 1u : 0u;
+}
+
 struct __align__(8) RowPart {
     float x, dxdy, y0, y1;  // before convert(): the segment
     float sign;
@@ -654,8 +756,8 @@ struct __align__(8) RowPart {
 __global__ void __launch_bounds__(TSF_NT, 3) k_tile_fill_segs(const float4* __restrict__ segs, uint32_t n_segs,
                                                               uint32_t grid_w, uint32_t grid_h, uint32_t width,
                                                               uint32_t height, int eo, uint8_t* __restrict__ coverage,
-                                                              uint32_t group_tiles,
-                                                              unsigned long long* __restrict__ n_records) {
+                                                              uint32_t group_tiles, TsfWork* __restrict__ work) {
+    if (work && work->leave) return;
     __shared__ RowPart part[TSF_CAP];
     __shared__ float area[TSF_TILES][TSF_NT];  // a warp's two pixel rows are its own
     __shared__ uint32_t counts[4 * TSF_NT / 32];
@@ -767,9 +869,9 @@ __global__ void __launch_bounds__(TSF_NT, 3) k_tile_fill_segs(const float4* __re
         const uint32_t px = t * TILE + tid % TILE;
         if (px < width && py < height) coverage[static_cast<size_t>(py) * width + px] = area_coverage(area[t - t0][tid], eo);
     }
-    if (g == 0 && n_records) {
+    if (g == 0 && work) {
         for (int o = 16; o; o >>= 1) records += __shfl_xor_sync(0xffffffffu, records, o);
-        if (lane == 0 && records) atomicAdd(n_records, records);
+        if (lane == 0 && records) atomicAdd(&work->records, records);
     }
 }
 
@@ -886,6 +988,10 @@ int check_segs(rrb_ctx* c, const rrb_buf* segs, uint32_t n) {
 // form, and the fill's chain per record is the shorter one: 18,432 segments in 17
 // x 17 5,535 / 5,096, 5,760 in 40 x 30 357 / 453.
 constexpr uint32_t kTileScanSegs = 1u << 15;
+// Segments from which the contents are looked at too (k_tile_load). With 2,048
+// the scan was never behind by more than a tenth whatever they were; 4,096 to
+// 8,192 is where long or crowded ones turn.
+constexpr uint32_t kTileLook = 4096;
 constexpr bool tile_scan_pays(uint32_t n, uint64_t row_ctas, uint64_t tiles) {
     return n <= kTileScanSegs && n <= 4096 * tiles && n * row_ctas <= (48ull << 20) + 300 * tiles;
 }
@@ -1063,18 +1169,24 @@ int rrb_record_tile_fill_segs(rrb_ctx* c, const rrb_aa_fill_params* p, uint64_t*
     while (group_tiles > 1 && ctas(group_tiles) < static_cast<uint64_t>(sm)) group_tiles /= 2;
     const uint64_t row_ctas = ctas(group_tiles);
     if (tile_scan_pays(n, row_ctas, tiles) && row_ctas <= 0x7FFFFFFFull && n * (2ull * gh + gw) < (1ull << 31)) {
-        if ((rc = rrb_ctx_fill_scratch(c, 0, 8, &v_off))) return rc;
-        auto* count = static_cast<unsigned long long*>(v_off);
-        if (n_records) FILL_CUDA(c, cudaMemsetAsync(count, 0, 8, s));
+        const bool look = n > kTileLook;
+        TsfWork* work = nullptr;
+        if (look || n_records) {
+            if ((rc = rrb_ctx_fill_scratch(c, 0, sizeof(TsfWork), &v_off))) return rc;
+            work = static_cast<TsfWork*>(v_off);
+            if (!look) FILL_CUDA(c, cudaMemsetAsync(work, 0, sizeof(TsfWork), s));
+            else k_tile_load<<<1, TL_THREADS, 0, s>>>(segs, n, gw, gh, p->height, (gw + group_tiles - 1) / group_tiles, work);
+        }
         k_tile_fill_segs<<<static_cast<unsigned>(row_ctas), TSF_NT, 0, s>>>(
             segs, n, gw, gh, p->width, p->height, p->fill_rule != 0,
-            static_cast<uint8_t*>(rrb_device_ptr(p->coverage)), group_tiles, n_records ? count : nullptr);
+            static_cast<uint8_t*>(rrb_device_ptr(p->coverage)), group_tiles, work);
         FILL_CUDA(c, cudaGetLastError());
-        if (n_records) {
-            FILL_CUDA(c, cudaMemcpyAsync(n_records, count, 8, cudaMemcpyDeviceToHost, s));
-            FILL_CUDA(c, cudaStreamSynchronize(s));
+        TsfWork done{};
+        if (work && (rc = rrb_ctx_read(c, work, sizeof done, &done))) return rc;
+        if (!done.leave) {
+            if (n_records) *n_records = done.records;
+            return RRB_OK;
         }
-        return RRB_OK;
     }
     if ((rc = rrb_ctx_fill_scratch(c, 0, 8ull * (n + 1), &v_off))) return rc;
     auto* off = static_cast<unsigned long long*>(v_off);
