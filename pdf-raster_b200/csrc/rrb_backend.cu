@@ -311,9 +311,11 @@ bool valid_tile(uint32_t w, uint32_t h) {
 // The kernels a resident batch's trials choose between, loaded when the
 // context is made: with CUDA's lazy module loading the first launch of a
 // kernel also loads it, and that time would land inside the first trial
-// render that uses it, making that tile or row shape look slower.
-void preload_trial_kernels() {
+// render that uses it, making that tile or row shape look slower. Returns the
+// first error of the settings that the row stage's launches depend on.
+cudaError_t preload_trial_kernels() {
     cudaFuncAttributes a{};
+    cudaError_t first = cudaSuccess;
 #define RRB_PRELOAD(...) cudaFuncGetAttributes(&a, reinterpret_cast<const void*>(__VA_ARGS__))
 #define RRB_PRELOAD_COMP(TW, TH)                      \
     do {                                              \
@@ -326,8 +328,10 @@ void preload_trial_kernels() {
     RRB_PRELOAD_COMP(128, 16);
     RRB_PRELOAD_COMP(128, 32);
     // The row stage's shared memory exceeds the 48 KB that need no asking.
-    auto rows_smem = [](auto kernel, size_t bytes) {
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+    auto rows_smem = [&](auto kernel, size_t bytes) {
+        const cudaError_t e =
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+        if (first == cudaSuccess) first = e;
     };
     rows_smem(k_rows<KCAP, ROWS_WARPS>, rows_smem_bytes<KCAP, ROWS_WARPS>());
     rows_smem(k_rows<KCAP_WIDE, 4>, rows_smem_bytes<KCAP_WIDE, 4>());
@@ -342,6 +346,7 @@ void preload_trial_kernels() {
 #undef RRB_PRELOAD_COMP
 #undef RRB_PRELOAD
     cudaGetLastError();
+    return first;
 }
 
 int launch_composite(rrb_ctx* c, int tw, int th, int grid, const PathInfo* info, const PageGeom* geom,
@@ -1932,14 +1937,15 @@ int rrb_init(int device, uint64_t mem_budget_bytes, rrb_ctx** out) {
         return RRB_ERR_DEVICE;
     }
     e = cudaMallocHost(reinterpret_cast<void**>(&c->h_read), 4096);
+    if (e == cudaSuccess) e = preload_trial_kernels();
     if (e != cudaSuccess) {
+        if (c->h_read) cudaFreeHost(c->h_read);
         cudaStreamDestroy(c->stream);
         delete c;
         return RRB_ERR_DEVICE;
     }
     c->tmp_batch = new rrb_batch();
     c->wave_batch = new rrb_batch();
-    preload_trial_kernels();
     c->tuning.tile_w = 64;
     c->tuning.tile_h = 16;
     c->tuning.rows_per_chunk = 32;
