@@ -455,7 +455,9 @@ typedef struct {
                                                in neither of the last two, nor in nonterminating_rows) */
     uint64_t tiles, tile_pairs;             /* tiles with work, (tile, path) pairs */
     uint64_t nonterminating_rows;           /* rows whose winding never returns to 0 */
-    uint64_t kernel_launches;               /* kernels launched by the last record call */
+    uint64_t kernel_launches;               /* kernels of the pipeline launched by the last record call, abandoned
+                                               attempts included; without the copies of a few bytes between the
+                                               host and the device (geometry, sizes), which may be kernels too */
     uint64_t scratch_grows;                 /* scratch buffers the call had to (re)allocate */
     uint64_t waves;                         /* page groups the batch was rendered in */
     uint64_t host_ns;                       /* host time of the call before its first kernel: validation,
