@@ -118,6 +118,9 @@ const AaJitter& jitter_by_y() {
 // Work per row: 64 x crossings + width, instead of 64 x width x
 // log(crossings). Crossings right of the chunk only shift its winding, those
 // left of it count for no pixel: neither is stored.
+// Two CTAs an SM: AaShared is 81,184 bytes (three, which 40 registers with 28
+// bytes of spills were compiled for, never fitted: calls 41.9 -> 41.1 and 50.8 ->
+// 49.0 us).
 // Measured: 48 glyph outlines (13,844 segments) in a 1,024 x 1,024 window 616
 // -> 36 us; 6 outlines (1,344 segments) in 2,047 x 2,050, even-odd, 960 -> 44
 // us (1 byte a pixel is 95 GB/s there). What is left is latency and barriers
@@ -153,6 +156,8 @@ struct AaShared {
     uint32_t plan, plan_c;  // see k_aa_fill
 };
 
+static_assert(2 * (sizeof(AaShared) + 1024) <= 228 * 1024, "two CTAs an SM");
+
 // Sample x of pixel px for sample offset jx, rounded as aa_fill_cpu does.
 __host__ __device__ __forceinline__ float aa_sample_x(uint32_t px, float jx) {
     return (static_cast<float>(px) + 0.5f + jx) - 0.5f;
@@ -170,7 +175,7 @@ __host__ __device__ __forceinline__ uint32_t aa_pixels_left(float xi, float jx, 
     return p;
 }
 
-__global__ void __launch_bounds__(AA_NT, 3) k_aa_fill(const float4* __restrict__ segs, uint32_t n_segs,
+__global__ void __launch_bounds__(AA_NT, 2) k_aa_fill(const float4* __restrict__ segs, uint32_t n_segs,
                                                       uint32_t width, uint32_t height, int eo,
                                                       const __grid_constant__ AaJitter J,
                                                       uint8_t* __restrict__ coverage) {
