@@ -534,7 +534,10 @@ int rrb_server_destroy(rrb_server* s);
  * NULL. Features and predictions (rrb_page_features_all, rrb_mlp_predict_host:
  * host work only) are computed by predict_threads host threads between submit
  * and the queue, so submitting stays cheap. Set the model before submitting
- * requests. */
+ * requests. The model and table that come with the package (cost_model.npz) were
+ * fitted to earlier kernels: on the present ones arrival order with 64x16 tiles
+ * (no model set) completes more pages at every offered rate measured, 585 a second
+ * against 528 to 540 at 2,000 offered. Fit them again (rrb.autotune) before use. */
 #define RRB_SCHED_SHORTEST_FIRST 1u
 #define RRB_SCHED_TILE_BY_MODEL 2u
 typedef struct {

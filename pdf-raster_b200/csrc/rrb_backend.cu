@@ -52,7 +52,12 @@ constexpr int KCAP_WIDE = 16;   // the same for the 4-warp row-stage shapes
 constexpr int kRowShapes = 5;
 constexpr uint64_t kLaneCountCurves = 1ull << 22;  // big curves whose lane counts are kept (128 MiB)
 constexpr uint32_t kLongWalk = 64;    // path points from which a warp walks a path
-constexpr uint64_t kFewPaths = 4096;  // paths up to which warps walk them all (one launch)
+// Paths up to which warps walk them all: one launch instead of two. Walk stage in
+// us, warps for all / a thread each for the short ones (5 points | 24 points):
+// 256 to 1,024 paths 16 / 20 | 16 / 22, 4,096 21 / 24 | 21 / 27, 16,384 36 / 35 |
+// 41 / 42, 65,536 64 / 48 | 74 / 63, 262,144 196 / 102. Paths of 64 points and
+// more have a warp either way and gain the launch, 8 us, at any number.
+constexpr uint64_t kFewPaths = 4096;
 constexpr uint64_t kMaxGroups = 0x3FFFFFFF;  // pixel rows (groups of four AA rows) of a wave's paths
 constexpr uint64_t kMaxRuns = 0x7FFFFFFF;    // row runs of its rectilinear paths and hairlines
 constexpr int SUPER = 256;      // supertile edge in pixels (a multiple of every tile shape)
@@ -678,15 +683,20 @@ int batch_upload(rrb_ctx* c, const rrb_path_batch_params* h, rrb_batch* B, const
     return RRB_OK;
 }
 
-// A batch uploaded per call with up to this many points is first launched whole, without waiting for a size: each stage reads its counts on the device,
-// the buffers that a count sizes are taken as the context's earlier renders left
+// A batch uploaded per call with up to this many points is first launched whole,
+// without waiting for a size: each stage reads its counts on the device, the
+// buffers that a count sizes are taken as the context's earlier renders left
 // them, and a count beyond its buffer stops every later stage before it touches
 // anything (BatchCounters::err; the pages are only written by the last). The
 // sizes come back behind the launches and are checked as they arrive; where one
 // did not fit, the batch is rendered again with the sizes read back between the
 // stages, which grows the buffers. Six waits of 10-15 us with the device idle
 // become none, calls of one glyph 304 -> 198 us, of 40 paths 475 -> 370, of 900
-// paths under clips 812 -> 692. Larger batches gain nothing by it.
+// paths under clips 812 -> 692. What it saves is some 40 us whatever the size,
+// while the buffers that hold bounds take 65 bytes a point: by size / whole, glyphs
+// in page-locked arrays, 0.11 M points 387 / 348 us, 0.87 M 832 / 788, 1.98 M
+// 1,491 / 1,450, 2.85 M 2,020 / 1,947, 3.72 M 2,530 / 2,489. At the limit that is
+// 3% of the call for 130 MB; from 4 Mi points on such batches are streamed.
 constexpr uint64_t kFreePoints = 2ull << 20;
 
 void release_scratch(rrb_ctx* c);

@@ -12,7 +12,8 @@
 //   k_rows          fill_intersections + write_intersect merge + per-row sort
 //                   + render_aa_line winding walk (scanner/mod.rs:393-642),
 //                   one warp per 32 AA rows of one path
-//   k_rows_slow     the same for rows whose merged list exceeds shared memory
+//   k_groups_mid    the same for pixel rows whose lists pass k_rows' capacity, a
+//   k_groups_slow   warp per row; _slow with the lists in global memory
 //   k_composite     draw_aa_line coverage + AA_GAMMA + render_span_aa div255
 //                   source-over (fill/mod.rs:344-401, pipe/aa.rs:192-208),
 //                   one CTA per page tile, paths in index order

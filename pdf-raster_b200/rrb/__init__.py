@@ -532,7 +532,8 @@ class Server:
         return out
 
     def set_cost_model(self, model=None, table=None, shortest_first=True, tile_by_model=True):
-        """Scheduler policy from a trained rrb.autotune.CostModel (or only its table)."""
+        """Scheduler policy from a trained rrb.autotune.CostModel (or only its table). The model that comes with
+        the package was fitted to earlier kernels and loses to the default, arrival order with 64x16 tiles."""
         keep = []
 
         def f32(a):
