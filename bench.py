@@ -117,7 +117,7 @@ class Clocks:
 # the glyph page reduced to 30,000 paths (10,979,156 segments, edge records
 # larger than L2), scaled to a full launch by its segment count.
 GLYPH_DRAM_BYTES_PER_SEGMENT = {
-    "rows": (387_725_568 + 43_464_192) / 10_979_156,
+    "rows": (388_048_896 + 44_584_960) / 10_979_156,
 }
 
 
