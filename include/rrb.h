@@ -218,7 +218,7 @@ int rrb_record_tile_fill(rrb_ctx* ctx, const rrb_tile_fill_params* p);
 /* tile_fill from segments: the tile records are those of build_tile_records
  * (crates/gpu/src/fill.rs:82-264, with a stable key sort), formed on the
  * device. *n_records (optional) receives their count: the call then waits on
- * the stream once. More than 4,096 segments: once or twice in any case, to
+ * the stream, once or twice, as with more than 4,096 segments in any case: to
  * choose between two ways by their contents and to size the records, which are
  * kept in the context's scratch. */
 int rrb_record_tile_fill_segs(rrb_ctx* ctx, const rrb_aa_fill_params* p, uint64_t* n_records);

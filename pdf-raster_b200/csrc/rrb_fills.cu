@@ -24,8 +24,8 @@
 // treated as empty instead of being read out of bounds.
 //
 // record_tile_fill_segs takes the same segments as aa_fill: where that is the
-// faster way (tile_scan_pays) they go straight to coverage (k_tile_fill_segs);
-// more of them, or larger windows, build the records on the
+// faster way (tile_scan_pays by the sizes, tile_look by the contents) they go
+// straight to coverage (k_tile_fill_segs); otherwise the records are built on the
 // device (build_tile_records, fill.rs:82-264: count, write in segment order,
 // stable radix sort by tile key, per-tile ranges by binary search), then run
 // tile_fill. Neither builds or uploads records on the host.
@@ -653,104 +653,8 @@ constexpr int TSF_NT = 256, TSF_TILES = 16, TSF_CAP = 1024;
 static_assert(TSF_NT == TF_THREADS && TSF_CAP == 4 * TSF_NT, "a pixel of a tile per thread, four segments at a time");
 struct TsfWork {
     unsigned long long records;  // of all tile rows
-    uint32_t leave, pad;         // the sorted records are the faster way (k_tile_load): nothing is written
+    uint32_t leave, pad;         // the sorted records are the faster way (tile_look): what is written does not count
 };
-
-// Whether the contents are for the scan, by one CTA before it. Where some tile
-// rows have many records the chain of their CTAs is the scan's time (0.6 to 1 us
-// for each that all eight warps walk; 1.05 ns of the whole chip for each record
-// and tile), while the sorted records cost 0.7 ns each and a chain of 0.19 to
-// 0.35 us in their tile. So a sample of the segments is added up by tile row, each as
-// its pairs of pixel rows x tiles in a row, assumed even over the row's groups.
-// Scan / sorted records in us: 1,024 x 1,024, 32,768 long segments 3,293 /
-// 1,142, 8,192 860 / 434; all in 28 pixel rows of it, 32,768 884 / 220, 8,192 247 /
-// 134; 2,048 x 2,048, 32,768 long ones 2,957 / 2,033. With the look, whole calls:
-// 1,164, 457, 240, 156 and 2,061; 14,752 short ones 70 -> 65. It costs 5 us,
-// won back by reading its answer with the count; a call that leaves pays for the
-// wait too.
-constexpr uint32_t TL_THREADS = 512;  // and entries of the load, a tile row (or 2^shift of them) each
-constexpr uint32_t TL_PICKS = 2;       // segments looked at per thread
-__global__ void __launch_bounds__(TL_THREADS) k_tile_load(const float4* __restrict__ segs, uint32_t n_segs, uint32_t grid_w,
-                                                          uint32_t grid_h, uint32_t height, uint32_t groups,
-                                                          TsfWork* __restrict__ work) {
-    __shared__ uint32_t step[TL_THREADS + 1];  // load of an entry, less that of the one before
-    __shared__ uint32_t part[TL_THREADS / 32], peaks[TL_THREADS / 32];
-    __shared__ float2 recs_of[TL_THREADS / 32];
-    const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    // Each pick is one out of `per` consecutive segments and stands for them all: those of
-    // an outline lie in the same rows, where all of them would add to the same
-    // words in turn (13 us of 14,000 segments).
-    const uint32_t per = (n_segs + TL_PICKS * TL_THREADS - 1) / (TL_PICKS * TL_THREADS), picks = n_segs / per;
-    float4 s[TL_PICKS];
-#pragma unroll
-    for (uint32_t j = 0; j < TL_PICKS; ++j) {
-        const uint32_t i = tid + j * TL_THREADS;
-        s[j] = i < picks ? segs[i * per + __umulhi(i * 2654435761u, per)] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
-    uint32_t shift = 0;
-    while (((grid_h - 1) >> shift) >= TL_THREADS) ++shift;
-    step[tid] = 0;
-    if (tid == 0) step[TL_THREADS] = 0;
-    __syncthreads();
-    float recs = 0.0f, walked = 0.0f;  // records; pairs of pixel rows that they touch
-    const float bottom = static_cast<float>(height), wide = static_cast<float>(min(grid_w, 255u));
-#pragma unroll
-    for (uint32_t j = 0; j < TL_PICKS; ++j) {
-        const float y0 = fmaxf(fminf(s[j].y, s[j].w), 0.0f), y1 = fminf(fmaxf(s[j].y, s[j].w), bottom);
-        if (!(y0 < y1)) continue;
-        const uint32_t r0 = min(static_cast<uint32_t>(y0) / TILE, grid_h - 1);
-        const uint32_t r1 = min(static_cast<uint32_t>(y1) / TILE, grid_h - 1);
-        const float tiles = fminf(fabsf(s[j].z - s[j].x) / fmaxf(fabsf(s[j].w - s[j].y), static_cast<float>(TILE)) + 1.0f, wide);
-        const uint32_t rows = r1 - r0 + 1;
-        // Pairs of pixel rows (a warp each) in a tile row: the mean of its rows.
-        const uint32_t pairs = (static_cast<uint32_t>(ceilf(0.5f * y1)) - static_cast<uint32_t>(0.5f * y0) + rows - 1) / rows;
-        recs += tiles * static_cast<float>(rows);
-        walked += tiles * static_cast<float>(rows * pairs);
-        uint32_t load = static_cast<uint32_t>(static_cast<float>(pairs) * tiles + 0.5f);
-        if (shift) load = max(1u, (load * min(rows, 1u << shift)) >> shift);  // the mean of the entry's rows
-        atomicAdd(&step[r0 >> shift], load);
-        atomicAdd(&step[(r1 >> shift) + 1], 0u - load);
-    }
-    __syncthreads();
-    uint32_t incl = step[tid];
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (static_cast<int>(lane) >= o) incl += t;
-    }
-    for (int o = 16; o; o >>= 1) {
-        recs += __shfl_xor_sync(0xffffffffu, recs, o);
-        walked += __shfl_xor_sync(0xffffffffu, walked, o);
-    }
-    if (lane == 31) part[w] = incl;
-    if (lane == 0) recs_of[w] = make_float2(recs, walked);
-    __syncthreads();
-    incl += __reduce_add_sync(0xffffffffu, lane < w ? part[lane] : 0u);
-    incl = __reduce_max_sync(0xffffffffu, incl);
-    if (lane == 0) peaks[w] = incl;
-    __syncthreads();
-    if (w) return;
-    const bool has = lane < TL_THREADS / 32;
-    const uint32_t peak = __reduce_max_sync(0xffffffffu, has ? peaks[lane] : 0u);
-    const float2 t = has ? recs_of[lane] : make_float2(0.0f, 0.0f);
-    float total = t.x;
-    walked = t.y;
-    for (int o = 16; o; o >>= 1) {
-        total += __shfl_xor_sync(0xffffffffu, total, o);
-        walked += __shfl_xor_sync(0xffffffffu, walked, o);
-    }
-    if (lane) return;
-    const float n = static_cast<float>(n_segs), of = n / static_cast<float>(picks);
-    const float tiles = static_cast<float>(grid_w) * static_cast<float>(grid_h);
-    const float row = of * static_cast<float>(peak) / 8.0f;  // records of the fullest row that a warp walks
-    // In its tile a sorted record is looked at by every warp: 0.19 us of the chain, 0.35 if all walk it.
-    const float in_tile = fmaxf(350.0f, 1520.0f * total / fmaxf(walked, 1.0f));
-    total *= of;
-    const float scan = 2.1e-3f * n * static_cast<float>(grid_h) * static_cast<float>(groups) + 0.5f * tiles +
-                       fmaxf(750.0f * row / static_cast<float>(groups), 1.05f * total);
-    const float sorted = 1e5f + 2.2f * n + tiles + 0.7f * total + in_tile * row / static_cast<float>(grid_w);
-    work->records = 0;
-    work->leave = scan > 1.15f * sorted + 2e4f ? 1u : 0u;
-}
 
 struct __align__(8) RowPart {
     float x, dxdy, y0, y1;  // before convert(): the segment
@@ -758,17 +662,142 @@ struct __align__(8) RowPart {
     uint32_t tx;            // first tile | last tile << 16
 };
 
+// Whether the contents are for the scan. Where a tile row, or a part of one, has
+// many records the chain of its CTA is the scan's time, and many records in all cost
+// it more of the whole chip than the sort. So a sample of the segments is added up by
+// the CTAs that they would load: tile rows x groups of tiles in `cells`, with the
+// rows' listed segments behind them.
+// In ns, fitted to 792 contents of 400 to 32,000 segments (short, long, upright, flat,
+// crowded in rows, in columns, in both) in windows from 64 x 64 to 5,000 x 6,000:
+//   scan: 320 for a hit of the busiest warp's two pixel rows and 176 for each further
+//   tile of it, 7 for a listed segment; or 0.88 for each record of all;
+//   sorted records: sort_call (what the call costs more than the scan's) and 46,000
+//   beyond 5,000 records, 2 a segment, 0.45 a tile, 920 for each record of the mean
+//   segment (a thread writes them one after another), 0.8 of the scan's chain in the
+//   fullest tile; or 0.6 for each record of all.
+// The records are asked for beyond `margin` times their estimate.
+// Whole calls, scan / sorted records / as chosen, in us: 917 x 1,341, 4,096 segments
+// around 14 pixel rows 521 / 151 / 201, 2,000 269 / 131 / 179; 3,000 x 100, a tenth of
+// both sides full, 6,000 741 / 196 / 215, 12,000 1,394 / 341 / 332; 1,024 x 1,024, long
+// ones, 4,096 447 / 292 / 359, 8,192 854 / 433 / 467, 32,768 3,311 / 1,139 / 1,165; all
+// in 28 pixel rows of it, 9,000 356 / 142 / 165; short ones all over it, 14,752 50 /
+// 135 / 54, 3,000 32 / 77 / 32.
+constexpr uint32_t TL_MIN = 512;     // segments from which it is worth asking (511 in 14 pixel rows: 85 / 69)
+constexpr uint32_t TL_CTAS = 1000;   // CTAs of a scan up to which it is asked beside it
+constexpr uint32_t TL_ROWS = 6;      // tile rows looked at per segment
+constexpr uint32_t TL_CELLS = TSF_TILES * TSF_NT;
+template <uint32_t NT, uint32_t PICKS>  // threads of the block, segments looked at
+__device__ __forceinline__ void tile_look(const float4* __restrict__ segs, uint32_t n_segs, uint32_t grid_w,
+                                          uint32_t grid_h, uint32_t height, uint32_t group_tiles, uint32_t* cells,
+                                          float sort_call, float margin, TsfWork* __restrict__ work) {
+    __shared__ float all_of[NT / 32];
+    __shared__ uint32_t peaks[NT / 32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const uint32_t groups = (grid_w + group_tiles - 1) / group_tiles;
+    // Large windows: 2^rs rows and 2^gs groups a cell, and their mean.
+    uint32_t rs = 0, gs = 0;
+    while (static_cast<uint64_t>(((groups - 1) >> gs) + 2) * (((grid_h - 1) >> rs) + 1) > TL_CELLS) {
+        if ((grid_h >> rs) >= (groups >> gs)) ++rs;
+        else ++gs;
+    }
+    const uint32_t cols = ((groups - 1) >> gs) + 2;  // the last: listed segments
+    const uint32_t wide = group_tiles << gs;
+    const uint32_t n_cells = cols * (((grid_h - 1) >> rs) + 1);
+    for (uint32_t i = tid; i < n_cells; i += NT) cells[i] = 0;
+    __syncthreads();
+    const uint32_t per = (n_segs + PICKS - 1) / PICKS, picks = n_segs / per;
+    float recs = 0.0f;
+    const float bottom = static_cast<float>(height);
+#pragma unroll 1
+    for (uint32_t i = tid; i < picks; i += NT) {
+        // One out of `per` consecutive segments stands for them all.
+        const uint32_t hash = i * 2654435761u;
+        const float4 q = segs[i * per + __umulhi(hash, per)];
+        const bool up = q.y > q.w;
+        const float x0 = up ? q.z : q.x, y0 = up ? q.w : q.y;
+        const float e0 = fmaxf(y0, 0.0f), e1 = fminf(up ? q.y : q.w, bottom);
+        const float slope = __fdividef(q.z - q.x, q.w - q.y);
+        if (!(e0 < e1) || !(fabsf(slope) < 1e30f)) continue;
+        const uint32_t r0 = min(static_cast<uint32_t>(e0) / TILE, grid_h - 1);
+        const uint32_t r1 = min(static_cast<uint32_t>(e1) / TILE, grid_h - 1);
+        // One out of `step` rows, from a row of its own on: else those of long
+        // segments that start in the same rows would meet in the same cells.
+        const uint32_t step = (r1 - r0) / TL_ROWS + 1;
+        for (uint32_t r = r0 + __umulhi(hash, step); r <= r1; r += step) {
+            const float a = fmaxf(e0, static_cast<float>(r * TILE)), b = fminf(e1, static_cast<float>(r * TILE + TILE));
+            if (!(a < b)) continue;
+            uint32_t* row = cells + (r >> rs) * cols;
+            atomicAdd(&row[cols - 1], step);
+            const float xa = x0 + slope * (a - y0), xb = x0 + slope * (b - y0);
+            const float lo = fminf(xa, xb) / TILE, hi = fmaxf(xa, xb) / TILE;
+            if (!(hi >= 0.0f && lo < static_cast<float>(grid_w))) continue;
+            const uint32_t ta = static_cast<uint32_t>(fmaxf(lo, 0.0f));
+            const uint32_t tb = static_cast<uint32_t>(fminf(hi, static_cast<float>(grid_w - 1)));
+            recs += static_cast<float>((tb - ta + 1) * step);
+            // Warps of the busiest row among those that it touches, in eighths.
+            const uint32_t pairs = static_cast<uint32_t>(ceilf(0.5f * b)) - static_cast<uint32_t>(0.5f * a);
+            const uint32_t load = step * min(8u, (8 * pairs + 2) / 5);
+            for (uint32_t g = ta / wide; g <= tb / wide; ++g) {
+                const uint32_t more = min(tb, g * wide + wide - 1) - max(ta, g * wide);
+                atomicAdd(&row[g], load * (20 + 11 * more));  // of 16 ns
+            }
+        }
+    }
+    __syncthreads();
+    uint32_t peak = 0;
+    for (uint32_t i = tid; i < n_cells; i += NT)
+        if (i % cols != cols - 1) peak = max(peak, 2 * cells[i] + 7 * cells[i - i % cols + cols - 1]);
+    peak = __reduce_max_sync(0xffffffffu, peak);
+    for (int o = 16; o; o >>= 1) recs += __shfl_xor_sync(0xffffffffu, recs, o);
+    if (lane == 0) {
+        all_of[w] = recs;
+        peaks[w] = peak;
+    }
+    __syncthreads();
+    if (tid) return;
+    for (uint32_t k = 1; k < NT / 32; ++k) {
+        recs += all_of[k];
+        peak = max(peak, peaks[k]);
+    }
+    const float n = static_cast<float>(n_segs), of = n / static_cast<float>(picks);
+    const float chain = of * static_cast<float>(peak) / static_cast<float>(1u << (rs + gs)), all = of * recs;
+    const float scan = fmaxf(chain, 0.88f * all);
+    const float tiles = static_cast<float>(grid_w) * static_cast<float>(grid_h);
+    const float sorted = sort_call + (all > 5000.0f ? 4.6e4f : 0.0f) + 2.0f * n + 0.45f * tiles + 920.0f * all / n +
+                         fmaxf(0.8f * chain / static_cast<float>(wide), 0.6f * all);
+    if (scan > margin * sorted) *const_cast<volatile uint32_t*>(&work->leave) = 1;
+}
+
+// The look by itself, before the scan.
+constexpr uint32_t TL_THREADS = 512;  // a segment each
+__global__ void __launch_bounds__(TL_THREADS) k_tile_look(const float4* __restrict__ segs, uint32_t n_segs, uint32_t grid_w,
+                                                      uint32_t grid_h, uint32_t height, uint32_t group_tiles,
+                                                      TsfWork* __restrict__ work) {
+    __shared__ uint32_t cells[TL_CELLS];
+    if (threadIdx.x == 0) *work = TsfWork{};
+    tile_look<TL_THREADS, TL_THREADS>(segs, n_segs, grid_w, grid_h, height, group_tiles, cells, 5.5e4f, 1.1f, work);
+}
+
+// LOOK: block 0 looks, the others scan meanwhile.
+template <bool LOOK>
 __global__ void __launch_bounds__(TSF_NT, 3) k_tile_fill_segs(const float4* __restrict__ segs, uint32_t n_segs,
                                                               uint32_t grid_w, uint32_t grid_h, uint32_t width,
                                                               uint32_t height, int eo, uint8_t* __restrict__ coverage,
                                                               uint32_t group_tiles, TsfWork* __restrict__ work) {
-    if (work && work->leave) return;
     __shared__ RowPart part[TSF_CAP];
     __shared__ float area[TSF_TILES][TSF_NT];  // a warp's two pixel rows are its own
+    if (LOOK && blockIdx.x == 0) {
+        tile_look<TSF_NT, 4 * TSF_NT>(segs, n_segs, grid_w, grid_h, height, group_tiles,
+                                      reinterpret_cast<uint32_t*>(&area[0][0]), 7.5e4f, 1.4f, work);
+        return;
+    }
+    if (!LOOK && work && work->leave) return;  // as k_tile_look left it
+    // LOOK: what block 0 has found by now.
+    auto left = [&]() { return LOOK && *const_cast<const volatile uint32_t*>(&work->leave) != 0; };
     __shared__ uint32_t counts[4 * TSF_NT / 32];
     const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const uint32_t groups = (grid_w + group_tiles - 1) / group_tiles;
-    const uint32_t ty = blockIdx.x / groups, g = blockIdx.x % groups;
+    const uint32_t cta = blockIdx.x - (LOOK ? 1 : 0), ty = cta / groups, g = cta % groups;
     const uint32_t t0 = g * group_tiles, t1 = min(grid_w, t0 + group_tiles);  // tiles of this CTA
     const float px_f = static_cast<float>(tid % TILE), py_f = static_cast<float>(tid / TILE);
     const float wy0 = 2.0f * static_cast<float>(w), wy1 = wy0 + 2.0f;     // this warp's rows
@@ -778,10 +807,16 @@ __global__ void __launch_bounds__(TSF_NT, 3) k_tile_fill_segs(const float4* __re
     uint32_t n = 0;                   // parts in the list
     unsigned long long records = 0;   // of this tile row (counted by the first group)
     auto walk = [&]() {
+        uint32_t since = 0;  // hits since the flag was last read
         for (uint32_t b = 0; b < n; b += 32) {
             const bool hit = b + lane < n && part[b + lane].y0 < wy1 && part[b + lane].y1 > wy0;
+            uint32_t m = __ballot_sync(0xffffffffu, hit);
+            if (LOOK && (since += __popc(m)) >= 32) {  // some 10 us
+                if (__any_sync(0xffffffffu, left())) return;
+                since = 0;
+            }
             // Four records' areas at a time (their chains overlap), added in order.
-            for (uint32_t m = __ballot_sync(0xffffffffu, hit); m;) {
+            while (m) {
                 float add[4];
                 bool on[4];
                 uint32_t at[4], t[4], e[4];
@@ -812,8 +847,10 @@ __global__ void __launch_bounds__(TSF_NT, 3) k_tile_fill_segs(const float4* __re
         }
     };
     // The listed segments' parts in this tile row, a segment a thread: packed
-    // first, so that no warp runs this for a lane or two.
-    auto convert = [&]() {
+    // first, so that no warp runs this for a lane or two. True where the sorted
+    // records are asked for: the block leaves as one.
+    auto convert = [&]() -> bool {
+        const bool gone = tid == 0 && left();
         for (uint32_t i = tid; i < n; i += TSF_NT) {
             const RowPart s = part[i];
             RowPart r{0.0f, 0.0f, 1.0f, 0.0f, 0.0f, 0u};  // reaches no row
@@ -825,7 +862,7 @@ __global__ void __launch_bounds__(TSF_NT, 3) k_tile_fill_segs(const float4* __re
             }
             part[i] = r;
         }
-        __syncthreads();
+        return __syncthreads_or(gone);
     };
     for (uint32_t base = 0; base < n_segs; base += TSF_CAP) {
         float4 s[4];
@@ -835,6 +872,7 @@ __global__ void __launch_bounds__(TSF_NT, 3) k_tile_fill_segs(const float4* __re
             const uint32_t k = base + u * TSF_NT + tid;
             if (k < n_segs) s[u] = segs[k];
         }
+        const bool gone = base == 0 && tid == 0 && left();  // with the loads above
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             // Off the tile row for certain (a NaN stays; convert() drops it).
@@ -843,7 +881,7 @@ __global__ void __launch_bounds__(TSF_NT, 3) k_tile_fill_segs(const float4* __re
             m[u] = __ballot_sync(0xffffffffu, !off);
             if (lane == 0) counts[u * (TSF_NT / 32) + w] = __popc(m[u]);
         }
-        __syncthreads();
+        if (__syncthreads_or(gone)) return;
         const uint32_t mine_n = counts[lane];  // four steps x eight warps
         uint32_t incl = mine_n;
 #pragma unroll
@@ -853,7 +891,7 @@ __global__ void __launch_bounds__(TSF_NT, 3) k_tile_fill_segs(const float4* __re
         }
         const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
         if (n + total > TSF_CAP) {  // the same for every thread
-            convert();
+            if (convert()) return;
             walk();
             n = 0;
             __syncthreads();
@@ -867,7 +905,7 @@ __global__ void __launch_bounds__(TSF_NT, 3) k_tile_fill_segs(const float4* __re
         n += total;
         __syncthreads();
     }
-    convert();
+    if (convert()) return;
     walk();
     const uint32_t py = ty * TILE + tid / TILE;
     for (uint32_t t = t0; t < t1; ++t) {
@@ -993,9 +1031,11 @@ int check_segs(rrb_ctx* c, const rrb_buf* segs, uint32_t n) {
 // form, and the fill's chain per record is the shorter one: 18,432 segments in 17
 // x 17 5,535 / 5,096, 5,760 in 40 x 30 357 / 453.
 constexpr uint32_t kTileScanSegs = 1u << 15;
-// Segments from which the contents are looked at too (k_tile_load). With 2,048
-// the scan was never behind by more than a tenth whatever they were; 4,096 to
-// 8,192 is where long or crowded ones turn.
+// Beyond this many segments the contents are looked at before the scan (3.5 us, and a
+// call that leaves has lost only that and a wait). Up to there the look runs beside
+// the scan's CTAs, which ask for its answer as they go: 2% or less with 256 CTAs,
+// 14% with 7,500 (hence TL_CTAS), and a call that leaves has lost some 45 us; and
+// only where the call waits for the count in any case.
 constexpr uint32_t kTileLook = 4096;
 constexpr bool tile_scan_pays(uint32_t n, uint64_t row_ctas, uint64_t tiles) {
     return n <= kTileScanSegs && n <= 4096 * tiles && n * row_ctas <= (48ull << 20) + 300 * tiles;
@@ -1173,16 +1213,17 @@ int rrb_record_tile_fill_segs(rrb_ctx* c, const rrb_aa_fill_params* p, uint64_t*
     auto ctas = [&](uint32_t t) { return static_cast<uint64_t>(gh) * ((gw + t - 1) / t); };
     while (group_tiles > 1 && ctas(group_tiles) < static_cast<uint64_t>(sm)) group_tiles /= 2;
     const uint64_t row_ctas = ctas(group_tiles);
-    if (tile_scan_pays(n, row_ctas, tiles) && row_ctas <= 0x7FFFFFFFull && n * (2ull * gh + gw) < (1ull << 31)) {
-        const bool look = n > kTileLook;
+    if (tile_scan_pays(n, row_ctas, tiles) && row_ctas < 0x7FFFFFFFull && n * (2ull * gh + gw) < (1ull << 31)) {
+        const bool look = n > kTileLook, beside = !look && n_records && n >= TL_MIN && row_ctas <= TL_CTAS;
         TsfWork* work = nullptr;
         if (look || n_records) {
             if ((rc = rrb_ctx_fill_scratch(c, 0, sizeof(TsfWork), &v_off))) return rc;
             work = static_cast<TsfWork*>(v_off);
             if (!look) FILL_CUDA(c, cudaMemsetAsync(work, 0, sizeof(TsfWork), s));
-            else k_tile_load<<<1, TL_THREADS, 0, s>>>(segs, n, gw, gh, p->height, (gw + group_tiles - 1) / group_tiles, work);
+            else k_tile_look<<<1, TL_THREADS, 0, s>>>(segs, n, gw, gh, p->height, group_tiles, work);
         }
-        k_tile_fill_segs<<<static_cast<unsigned>(row_ctas), TSF_NT, 0, s>>>(
+        const auto fill = beside ? k_tile_fill_segs<true> : k_tile_fill_segs<false>;
+        fill<<<static_cast<unsigned>(row_ctas) + (beside ? 1 : 0), TSF_NT, 0, s>>>(
             segs, n, gw, gh, p->width, p->height, p->fill_rule != 0,
             static_cast<uint8_t*>(rrb_device_ptr(p->coverage)), group_tiles, work);
         FILL_CUDA(c, cudaGetLastError());

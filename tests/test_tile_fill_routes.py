@@ -56,6 +56,11 @@ def _contents(kind, n, w, h):
     rng = np.random.default_rng(n)
     if kind == "long":
         return rng.uniform((-3, -3, -3, -3), (w + 3, h + 3, w + 3, h + 3), (n, 4)).astype(np.float32)
+    if kind == "short":
+        return _short(n, w, h, n)
+    if kind in ("line", "corner"):  # a line of text; a tenth of both sides
+        a = rng.uniform((0, 0), (w, 14) if kind == "line" else (w / 10, h / 10), (n, 2))
+        return np.concatenate([a, a + rng.normal(0, 1, (n, 2)) * ((60, 8) if kind == "line" else (8, 8))], 1).astype(np.float32)
     a = rng.uniform((0, 0), (w, 20), (n, 2))  # crowded: the first 28 pixel rows
     s = np.concatenate([a, a + rng.normal(0, 3, (n, 2))], 1).astype(np.float32)
     s[::97, 0], s[::89, 3] = np.nan, np.inf
@@ -63,17 +68,23 @@ def _contents(kind, n, w, h):
 
 
 @pytest.mark.parametrize("w,h,n,kind,by_records", [
-    (1024, 1024, 4096, "long", False), (1024, 1024, 9000, "long", True), (1024, 1024, 9000, "crowded", True),
-    (200, 200, 9000, "crowded", False), (3000, 1200, 30000, "long", True), (40, 17000, 20000, "crowded", True)])
+    (1024, 1024, 4096, "long", True), (1024, 1024, 9000, "long", True), (1024, 1024, 9000, "crowded", True),
+    (200, 200, 9000, "crowded", False), (3000, 1200, 30000, "long", True), (40, 17000, 20000, "crowded", True),
+    # Crowded in columns too, and few: seen beside the scan from 512 segments on, before it from 4,097.
+    (917, 1341, 4097, "line", True), (917, 1341, 4096, "line", True), (917, 1341, 2000, "line", True),
+    (917, 1341, 511, "line", False), (3000, 100, 6000, "corner", True), (3000, 100, 3000, "corner", True),
+    (3000, 100, 2000, "crowded", None), (16, 16, 513, "long", None), (1, 1, 600, "crowded", None),
+    # Cells of eight tile rows, and of two groups of tiles.
+    (1024, 1024, 3000, "short", False), (8192, 8192, 5000, "short", False), (1048560, 16, 5000, "short", None)])
 def test_the_segments_choose_the_route(rrb_lib, oracle, w, h, n, kind, by_records):
-    """Up to 4,096 segments are not looked at. 17,000 pixel rows: two tile rows an entry of the look."""
+    """by_records: where the times of the two routes are well apart (None: either)."""
     segs = _contents(kind, n, w, h)
     recs, starts, counts, gw = oracle.build_tile_records(segs, 0.0, 0.0, w, h)
     for rule in (0, 1):
         with rrb_lib.B200Backend(0) as be:
             got, n_recs, used = _run(be, segs, w, h, rule)
         assert n_recs == len(recs)
-        assert (used >= 32 * n_recs) == by_records
+        assert by_records is None or (used >= 32 * n_recs) == by_records
         assert np.array_equal(got, oracle.tile_fill(recs, starts, counts, gw, w, h, eo=bool(rule)).ravel())
 
 
